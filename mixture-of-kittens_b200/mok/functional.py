@@ -15,6 +15,7 @@ Differences a caller can observe:
 """
 from __future__ import annotations
 
+import functools
 import os
 import math
 from dataclasses import dataclass
@@ -250,8 +251,11 @@ def clear_workspace_cache() -> None:
     _WORKSPACE_CACHE.clear()
 
 
+_device_properties = functools.cache(torch.cuda.get_device_properties)       # constant for the life of the process
+
+
 def _validate_config(config: MoKConfig, ws: MoKWorkspace) -> None:
-    props = torch.cuda.get_device_properties(ws.device)
+    props = _device_properties(ws.device)
     for label, value in (("fwd_num_comm_sms", config.fwd_num_comm_sms), ("bwd_num_comm_sms", config.bwd_num_comm_sms)):
         if type(value) is not int or value <= 0:
             raise ValueError(f"{label} must be a positive integer")

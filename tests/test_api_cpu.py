@@ -246,3 +246,60 @@ def test_bench_reference_arm_runs_on_rank_zero_only_and_c1_line(tmp_path):
     line = json.loads(c1.stdout.strip().splitlines()[-1])
     assert line["impl"] == "reference" and line["unit"] == "GFLOP/s" and line["steps"] >= 10
     assert line["cpu_baseline"]["cores"] >= 1 and line["value"] > 0
+
+
+def test_eager_operators_skip_the_dispatcher_only_where_it_would_forward_the_call():
+    """The short way into an operator body gives what the dispatcher gives (values, version bump of what it writes) and
+    is left whenever autograd, a mode, a transform, forward-mode AD, inexact argument types or keywords are involved."""
+    import mok
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    def scale_into(x: "Tensor", factor: "float | None", out: "Tensor", times: "int" = 1) -> None:
+        out.copy_(x * (1.0 if factor is None else factor) * times)
+    scale_into.__annotations__ = {"x": "Tensor", "factor": "float | None", "out": "Tensor", "times": "int"}
+    op = mok.ops._operator("mok_test::scale_into", mutates_args=("out",),
+                           schema="(Tensor x, float? factor, Tensor(a!) out, int times=1) -> ()")(scale_into)
+    x, out = torch.arange(4.0), torch.zeros(4)
+
+    def direct(*args):
+        return op._forwards_only(args)
+
+    assert direct(x, 2.0, out) and direct(x, None, out, 3)
+    before = out._version
+    op(x, 2.0, out, 3)
+    assert torch.equal(out, x * 6) and out._version > before
+    via = torch.zeros(4)
+    before = via._version
+    op(x=x, factor=2.0, out=via, times=3)                   # keywords: the dispatcher
+    assert torch.equal(via, out) and via._version > before
+    with torch.inference_mode():
+        inferred = torch.zeros(4)
+        op(x, 2.0, inferred)
+        assert torch.equal(inferred, x * 2)
+
+    needs_grad = torch.ones(4, requires_grad=True)
+    assert not direct(needs_grad, 2.0, out)
+    with torch.no_grad():
+        assert direct(needs_grad, 2.0, out)
+    assert not direct(x, 2.0, out, True) and not direct(x, 2.0) and not direct(x, "2", out)
+
+    class Subclass(torch.Tensor):
+        pass
+    assert not direct(x.as_subclass(Subclass), 2.0, out)
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+    seen = []
+    with Mode():
+        op(x, 2.0, out)
+    assert any("scale_into" in name for name in seen)
+    with torch.autograd.forward_ad.dual_level():
+        assert not direct(x, 2.0, out)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        op(x, 2.0, out)
+    assert any("scale_into" in e.key for e in prof.key_averages())
+    inside = []
+    torch.func.vmap(lambda row: inside.append(direct(row, 2.0, out)) or row)(torch.ones(2, 4))
+    assert inside == [False]
