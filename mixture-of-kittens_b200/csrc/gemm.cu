@@ -68,8 +68,7 @@ int device_sm_count() {
 
 namespace {
 template <int kA, int kB, int kEpi, bool kW, bool k2>
-int launch_inst(const CUtensorMap& a0, const CUtensorMap& b0, const CUtensorMap& a1, const CUtensorMap& b1, const GemmParams& p,
-                int grid, cudaStream_t stream) {
+int launch_inst(const GemmBatch& batch, int grid, cudaStream_t stream) {
     auto* kern = grouped_gemm_kernel<kA, kB, kEpi, kW, k2>;
     static bool configured[64] = {false};   // per instantiation and device: the attribute is sticky
     int dev = 0;
@@ -89,9 +88,9 @@ int launch_inst(const CUtensorMap& a0, const CUtensorMap& b0, const CUtensorMap&
         attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
-        MOK_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, a0, b0, a1, b1, p));
+        MOK_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, batch));
     } else {
-        kern<<<grid, kGemmThreads, kGemmSmemBytes, stream>>>(a0, b0, a1, b1, p);
+        kern<<<grid, kGemmThreads, kGemmSmemBytes, stream>>>(batch);
     }
     MOK_CUDA_CHECK(cudaGetLastError());
     return MOK_OK;
@@ -105,35 +104,43 @@ bool use_pairs() {
     return on;
 }
 
-int launch_grouped_gemm(int a_major, int b_major, int epi, bool wgrad, const GemmOperands& ops, const GemmParams& p,
-                        int max_tiles, int max_ctas, int prof_slot, cudaStream_t stream) {
-    if (max_tiles <= 0) return MOK_OK;
-    // the epilogues use 256-bit global accesses: 32-byte aligned tensors and row pitches
-    for (const void* ptr : {static_cast<const void*>(p.out0), static_cast<const void*>(p.out1), static_cast<const void*>(p.out2),
-                            static_cast<const void*>(p.in0), static_cast<const void*>(p.in1)})
-        if (reinterpret_cast<uintptr_t>(ptr) % 32 != 0) return MOK_ERR_INVALID;
-    if (p.ld_out % 16 != 0) return MOK_ERR_INVALID;
-    CUtensorMap a0, b0, a1, b1;
+int launch_grouped_gemm(int a_major, int b_major, int epi, bool wgrad, const GemmCall* calls, int num_calls, GemmBatch& batch,
+                        int max_ctas, int prof_slot, cudaStream_t stream) {
+    if (num_calls < 1 || num_calls > (wgrad ? kMaxGemms : 2)) return MOK_ERR_INVALID;
     // A: K-major box {64 K, 128 rows}; M-major box {64 M, 64 K-rows}
     const uint32_t a_box_outer = a_major == kMajorK ? kBlockM : kBlockK;
     // B: K-major box {64 K, 256 rows} (128 when the tile is split into gate|up halves); N-major box {64 N, 64 K-rows}
     const bool pairs = use_pairs();
     // (a CTA of a pair stages 128 rows of B, so its box is 128 rows too)
     const uint32_t b_box_outer = b_major == kMajorK ? ((epi == kEpiSwigluFwd || pairs) ? kBlockN / 2 : kBlockN) : kBlockK;
-    int rc;
-    if ((rc = make_tmap_2d(&a0, ops.a0, ops.a_inner, ops.a_outer, ops.a_inner * 2, 64, a_box_outer, 2))) return rc;
-    if ((rc = make_tmap_2d(&b0, ops.b0, ops.b_inner, ops.b_outer, ops.b_inner * 2, 64, b_box_outer, 2))) return rc;
-    if ((rc = make_tmap_2d(&a1, ops.a1 ? ops.a1 : ops.a0, ops.a_inner, ops.a_outer, ops.a_inner * 2, 64, a_box_outer, 2))) return rc;
-    if ((rc = make_tmap_2d(&b1, ops.b1 ? ops.b1 : ops.b0, ops.b_inner, ops.b_outer, ops.b_inner * 2, 64, b_box_outer, 2))) return rc;
+    int n = 0;
+    long long max_tiles = 0;
+    for (int i = 0; i < num_calls; ++i) {
+        const GemmParams& p = calls[i].p;
+        const GemmOperands& ops = calls[i].ops;
+        if (calls[i].max_tiles <= 0) continue;
+        // the epilogues use 256-bit global accesses: 32-byte aligned tensors and row pitches
+        for (const void* ptr : {static_cast<const void*>(p.out0), static_cast<const void*>(p.out1), static_cast<const void*>(p.out2),
+                                static_cast<const void*>(p.in0), static_cast<const void*>(p.in1)})
+            if (reinterpret_cast<uintptr_t>(ptr) % 32 != 0) return MOK_ERR_INVALID;
+        if (p.ld_out % 16 != 0) return MOK_ERR_INVALID;
+        MOK_TRY(make_tmap_2d(&batch.a0[n], ops.a0, ops.a_inner, ops.a_outer, ops.a_inner * 2, 64, a_box_outer, 2));
+        MOK_TRY(make_tmap_2d(&batch.b0[n], ops.b0, ops.b_inner, ops.b_outer, ops.b_inner * 2, 64, b_box_outer, 2));
+        if (ops.a1) MOK_TRY(make_tmap_2d(&batch.a1[n], ops.a1, ops.a_inner, ops.a_outer, ops.a_inner * 2, 64, a_box_outer, 2));
+        if (ops.b1) MOK_TRY(make_tmap_2d(&batch.b1[n], ops.b1, ops.b_inner, ops.b_outer, ops.b_inner * 2, 64, b_box_outer, 2));
+        batch.gemm[n++] = p;
+        // max_tiles counts 128-row tiles; a pair covers two of them
+        max_tiles += pairs ? ((calls[i].max_tiles + 1) / 2) * 2 : calls[i].max_tiles;
+    }
+    if (n == 0) return MOK_OK;
+    batch.num_gemms = n;
     int ctas = device_sm_count();
     if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;
-    // max_tiles counts 128-row tiles; a pair covers two of them
-    const int want = pairs ? ((max_tiles + 1) / 2) * 2 : max_tiles;
-    const int grid = want < ctas ? want : (pairs ? (ctas & ~1) : ctas);
+    const int grid = max_tiles < ctas ? static_cast<int>(max_tiles) : (pairs ? (ctas & ~1) : ctas);
     ProfScope prof(prof_slot, stream);
 #define MOK_INST(A, B, EPI, W)                                                              \
-    (pairs ? launch_inst<A, B, EPI, W, true>(a0, b0, a1, b1, p, grid, stream)              \
-           : launch_inst<A, B, EPI, W, false>(a0, b0, a1, b1, p, grid, stream))
+    (pairs ? launch_inst<A, B, EPI, W, true>(batch, grid, stream)                          \
+           : launch_inst<A, B, EPI, W, false>(batch, grid, stream))
 
     if (!wgrad && a_major == kMajorK && b_major == kMajorK && epi == kEpiStore)
         return MOK_INST(kMajorK, kMajorK, kEpiStore, false);
@@ -155,35 +162,32 @@ extern "C" int mok_gemm_bf16(const void* a, const void* b, void* c, int m, int n
     using namespace mok;
     if (!a || !b || !c || m <= 0 || n <= 0 || k <= 0) return MOK_ERR_INVALID;
     if (m % (2 * kBlockM) || n % kBlockN || k % kBlockK) return MOK_ERR_INVALID;
-    GemmParams p{};
-    p.num_tokens = nullptr;
-    p.capacity = 0;
-    p.row_offset = 0;
-    p.tokens_per_expert = nullptr;
-    p.num_experts = 1;
+    GemmBatch batch{};
+    batch.status = status;
+    GemmCall call{};
+    GemmParams& p = call.p;
+    GemmOperands& ops = call.ops;
     p.n_tiles = n / kBlockN;
     p.num_segs = 1;
     p.out0 = static_cast<__nv_bfloat16*>(c);
     p.ld_out = n;
-    p.status = status;
-    GemmOperands ops{};
     ops.a0 = a; ops.b0 = b;
     const bool wgrad = a_mn_major != 0;
     if (!wgrad) {
-        p.rows_host = m; p.row_limit = m;
+        p.rows_host = m;
         p.k_blocks_per_seg = k / kBlockK;
         ops.a_inner = k; ops.a_outer = m;
         if (b_mn_major) { ops.b_inner = n; ops.b_outer = k; p.b_rows_per_expert = k; }
         else { ops.b_inner = k; ops.b_outer = n; p.b_rows_per_expert = n; }
     } else {
         if (!b_mn_major) return MOK_ERR_UNSUPPORTED;
-        p.rows_host = k; p.row_limit = k;       // contraction runs over the rows of both operands
+        p.rows_host = k;                        // contraction runs over the rows of both operands
         p.m_tiles_w = m / kBlockM;
         p.out_expert_stride = 0;
         ops.a_inner = m; ops.a_outer = k;
         ops.b_inner = n; ops.b_outer = k;
     }
-    const int tiles = (m / kBlockM) * (n / kBlockN);
-    return launch_grouped_gemm(a_mn_major ? kMajorMN : kMajorK, b_mn_major ? kMajorMN : kMajorK, kEpiStore, wgrad, ops, p,
-                               tiles, 0, kSlotGemmTest, static_cast<cudaStream_t>(stream));
+    call.max_tiles = (m / kBlockM) * (n / kBlockN);
+    return launch_grouped_gemm(a_mn_major ? kMajorMN : kMajorK, b_mn_major ? kMajorMN : kMajorK, kEpiStore, wgrad, &call, 1, batch,
+                               0, kSlotGemmTest, static_cast<cudaStream_t>(stream));
 }

@@ -12,6 +12,7 @@
 #include <climits>
 #include <cmath>
 #include <cstdlib>
+#include <initializer_list>
 #include <mutex>
 #include <vector>
 
@@ -58,33 +59,39 @@ struct PassCtx {
     bool dedicated = false;        // the budget is SMs of the movers' own (fat CTAs), not mover CTAs beside the GEMM CTAs
 };
 
-GemmParams base_params(const mok_layer_common& c, const PassCtx& x, bool routed, int off, int limit) {
-    GemmParams p{};
-    if (routed) p.chunk = x.chunk;
-    if (routed) {
-        p.num_tokens = c.num_tokens;
-        p.capacity = c.schedule_capacity;
-        p.tokens_per_expert = c.tokens_per_expert;
-        p.num_experts = c.num_local_experts;
-        p.row_offset = off;
-        p.row_limit = limit;
-    } else {
-        p.rows_host = c.num_local_tokens;
-        p.row_limit = c.num_local_tokens;
-        p.num_experts = 1;
-    }
-    p.num_segs = 1;
-    p.limit = c.swiglu_limit;
-    p.has_limit = c.has_swiglu_limit;
-    p.status = c.status;
-    return p;
+// fields of a launch that covers `limit` schedule rows from `off` on (and, in a joint launch, the local tokens)
+GemmBatch gemm_batch(const mok_layer_common& c, const PassCtx& x, int off, int limit) {
+    GemmBatch g{};
+    g.chunk = x.chunk;
+    g.num_tokens = c.num_tokens;
+    g.capacity = c.schedule_capacity;
+    g.tokens_per_expert = c.tokens_per_expert;
+    g.num_experts = c.num_local_experts;
+    g.row_offset = off;
+    g.row_limit = limit;
+    g.limit = c.swiglu_limit;
+    g.has_limit = c.has_swiglu_limit;
+    g.status = c.status;
+    return g;
 }
 
+GemmCall gemm_call(const mok_layer_common& c, bool routed) {
+    GemmCall k{};
+    k.p.routed = routed ? 1 : 0;
+    k.p.rows_host = routed ? 0 : c.num_local_tokens;
+    k.p.num_segs = 1;
+    return k;
+}
+
+// A pass is a sequence of stages (gate|up, down, ...).  Each stage exists once for the dense shared expert on the local
+// tokens (`rows` = their number) and once for the routed experts on a window of schedule rows; the two have the same
+// kernel, so one launch can hold both (see launch_stage).
 
 // gate|up GEMM with fused SwiGLU: A [rows, H] K-major, B = (Wg, Wu) [E*I, H] K-major
-int run_gate_up(const mok_layer_common& c, const PassCtx& x, const Dims& d, bool routed, int off, int limit, const void* a, int a_rows,
-                const void* wg, const void* wu, void* gate, void* up, void* hidden, cudaStream_t s) {
-    GemmParams p = base_params(c, x, routed, off, limit);
+GemmCall gate_up(const mok_layer_common& c, const Dims& d, bool routed, int rows, const void* a, int a_rows,
+                 const void* wg, const void* wu, void* gate, void* up, void* hidden) {
+    GemmCall k = gemm_call(c, routed);
+    GemmParams& p = k.p;
     p.n_tiles = d.I / (kBlockN / 2);
     p.k_blocks_per_seg = d.H / kBlockK;
     p.b_rows_per_expert = d.I;
@@ -92,36 +99,37 @@ int run_gate_up(const mok_layer_common& c, const PassCtx& x, const Dims& d, bool
     p.out1 = static_cast<__nv_bfloat16*>(up);
     p.out2 = static_cast<__nv_bfloat16*>(hidden);
     p.ld_out = d.I;
-    GemmOperands o{};
+    GemmOperands& o = k.ops;
     o.a0 = a; o.b0 = wg; o.b1 = wu;
     o.a_inner = d.H; o.a_outer = a_rows;
     o.b_inner = d.H; o.b_outer = static_cast<uint64_t>(routed ? d.El : 1) * d.I;
-    return launch_grouped_gemm(kMajorK, kMajorK, kEpiSwigluFwd, false, o, p, (limit / kBlockM) * p.n_tiles, routed ? x.gemm_ctas : 0,
-                               routed ? kSlotGateUpRouted : kSlotGateUpShared, s);
+    k.max_tiles = (rows / kBlockM) * p.n_tiles;
+    return k;
 }
 
 // down GEMM: A = hidden [rows, I] K-major, B = Wd [E*H, I] K-major
-int run_down(const mok_layer_common& c, const PassCtx& x, const Dims& d, bool routed, int off, int limit, const void* hidden, int a_rows,
-             const void* wd, void* y, cudaStream_t s) {
-    GemmParams p = base_params(c, x, routed, off, limit);
+GemmCall down(const mok_layer_common& c, const Dims& d, bool routed, int rows, const void* hidden, int a_rows, const void* wd, void* y) {
+    GemmCall k = gemm_call(c, routed);
+    GemmParams& p = k.p;
     p.n_tiles = d.H / kBlockN;
     p.k_blocks_per_seg = d.I / kBlockK;
     p.b_rows_per_expert = d.H;
     p.out0 = static_cast<__nv_bfloat16*>(y);
     p.ld_out = d.H;
-    GemmOperands o{};
+    GemmOperands& o = k.ops;
     o.a0 = hidden; o.b0 = wd;
     o.a_inner = d.I; o.a_outer = a_rows;
     o.b_inner = d.I; o.b_outer = static_cast<uint64_t>(routed ? d.El : 1) * d.H;
-    return launch_grouped_gemm(kMajorK, kMajorK, kEpiStore, false, o, p, (limit / kBlockM) * p.n_tiles, routed ? x.gemm_ctas : 0,
-                               routed ? kSlotDownRouted : kSlotDownShared, s);
+    k.max_tiles = (rows / kBlockM) * p.n_tiles;
+    return k;
 }
 
 // d_hidden = d_y @ Wd (B is [E*H, I] read N-major), fused SwiGLU backward
-int run_dgrad_down(const mok_layer_common& c, const PassCtx& x, const Dims& d, bool routed, int off, int limit, const void* d_y, int a_rows,
-                   const void* wd, const void* gate, const void* up, void* d_hidden, void* d_gate, void* d_up,
-                   const float* row_scale, float* partials, cudaStream_t s) {
-    GemmParams p = base_params(c, x, routed, off, limit);
+GemmCall dgrad_down(const mok_layer_common& c, const Dims& d, bool routed, int rows, const void* d_y, int a_rows,
+                    const void* wd, const void* gate, const void* up, void* d_hidden, void* d_gate, void* d_up,
+                    const float* row_scale, float* partials) {
+    GemmCall k = gemm_call(c, routed);
+    GemmParams& p = k.p;
     p.n_tiles = d.I / kBlockN;
     p.k_blocks_per_seg = d.H / kBlockK;
     p.b_rows_per_expert = d.H;
@@ -133,50 +141,81 @@ int run_dgrad_down(const mok_layer_common& c, const PassCtx& x, const Dims& d, b
     p.ld_out = d.I;
     p.row_scale = row_scale;
     p.partials = partials;
-    GemmOperands o{};
+    GemmOperands& o = k.ops;
     o.a0 = d_y; o.b0 = wd;
     o.a_inner = d.H; o.a_outer = a_rows;
     o.b_inner = d.I; o.b_outer = static_cast<uint64_t>(routed ? d.El : 1) * d.H;
-    return launch_grouped_gemm(kMajorK, kMajorMN, kEpiSwigluBwd, false, o, p, (limit / kBlockM) * p.n_tiles, routed ? x.gemm_ctas : 0,
-                               routed ? kSlotDgradDownRouted : kSlotDgradDownShared, s);
+    k.max_tiles = (rows / kBlockM) * p.n_tiles;
+    return k;
 }
 
 // d_x = d_gate @ Wg + d_up @ Wu in one accumulator (B = [E*I, H] read N-major)
-int run_dgrad_gate_up(const mok_layer_common& c, const PassCtx& x, const Dims& d, bool routed, int off, int limit, const void* d_gate,
-                      const void* d_up, int a_rows, const void* wg, const void* wu, void* d_x, cudaStream_t s) {
-    GemmParams p = base_params(c, x, routed, off, limit);
+GemmCall dgrad_gate_up(const mok_layer_common& c, const Dims& d, bool routed, int rows, const void* d_gate,
+                       const void* d_up, int a_rows, const void* wg, const void* wu, void* d_x) {
+    GemmCall k = gemm_call(c, routed);
+    GemmParams& p = k.p;
     p.n_tiles = d.H / kBlockN;
     p.k_blocks_per_seg = d.I / kBlockK;
     p.num_segs = 2;
     p.b_rows_per_expert = d.I;
     p.out0 = static_cast<__nv_bfloat16*>(d_x);
     p.ld_out = d.H;
-    GemmOperands o{};
+    GemmOperands& o = k.ops;
     o.a0 = d_gate; o.a1 = d_up; o.b0 = wg; o.b1 = wu;
     o.a_inner = d.I; o.a_outer = a_rows;
     o.b_inner = d.H; o.b_outer = static_cast<uint64_t>(routed ? d.El : 1) * d.I;
-    return launch_grouped_gemm(kMajorK, kMajorMN, kEpiStore, false, o, p, (limit / kBlockM) * p.n_tiles, routed ? x.gemm_ctas : 0,
-                               routed ? kSlotDgradGateUpRouted : kSlotDgradGateUpShared, s);
+    k.max_tiles = (rows / kBlockM) * p.n_tiles;
+    return k;
 }
 
 // dW[e] [m, n] = A[rows_e, m]^T @ B[rows_e, n]; both operands are read MN-major straight from the
 // row-major activations
-int run_wgrad(const mok_layer_common& c, const PassCtx& x, bool routed, int off, int limit, const void* a, int m, const void* b, int n,
-              int rows, void* dw, int accumulate, cudaStream_t s) {
-    GemmParams p = base_params(c, x, routed, off, limit);
+GemmCall wgrad(const mok_layer_common& c, bool routed, const void* a, int m, const void* b, int n, int rows, void* dw, int accumulate) {
+    GemmCall k = gemm_call(c, routed);
+    GemmParams& p = k.p;
     p.m_tiles_w = m / kBlockM;
     p.n_tiles = n / kBlockN;
     p.out0 = static_cast<__nv_bfloat16*>(dw);
     p.ld_out = n;
     p.out_expert_stride = static_cast<long long>(m) * n;
     p.accumulate = accumulate;
-    GemmOperands o{};
+    GemmOperands& o = k.ops;
     o.a0 = a; o.b0 = b;
     o.a_inner = m; o.a_outer = rows;
     o.b_inner = n; o.b_outer = rows;
-    const int experts = routed ? c.num_local_experts : 1;
-    return launch_grouped_gemm(kMajorMN, kMajorMN, kEpiStore, true, o, p, experts * p.m_tiles_w * p.n_tiles, 0,
-                               routed ? kSlotWgradRouted : kSlotWgradShared, s);
+    k.max_tiles = (routed ? c.num_local_experts : 1) * p.m_tiles_w * p.n_tiles;
+    return k;
+}
+
+enum Stage { kStageGateUp, kStageDown, kStageDgradDown, kStageDgradGateUp, kStageWgrad };
+
+// One launch of a stage.  `calls` may hold shared-expert GEMMs, routed ones, or both (a joint launch, used on one
+// rank where the row movement does not run beside the shared expert).  A launch is booked under the routed slot as
+// soon as it holds routed rows.
+int launch_stage(Stage stage, std::initializer_list<GemmCall> calls, const mok_layer_common& c, const PassCtx& x, int off, int limit,
+                 cudaStream_t s) {
+    bool routed = false;
+    for (const GemmCall& k : calls) routed = routed || k.p.routed;
+    GemmBatch g = gemm_batch(c, x, off, limit);
+    if (!routed) g.num_experts = 0;
+    const int cap = routed && stage != kStageWgrad ? x.gemm_ctas : 0, n = static_cast<int>(calls.size());
+    switch (stage) {
+        case kStageGateUp:
+            return launch_grouped_gemm(kMajorK, kMajorK, kEpiSwigluFwd, false, calls.begin(), n, g, cap,
+                                       routed ? kSlotGateUpRouted : kSlotGateUpShared, s);
+        case kStageDown:
+            return launch_grouped_gemm(kMajorK, kMajorK, kEpiStore, false, calls.begin(), n, g, cap,
+                                       routed ? kSlotDownRouted : kSlotDownShared, s);
+        case kStageDgradDown:
+            return launch_grouped_gemm(kMajorK, kMajorMN, kEpiSwigluBwd, false, calls.begin(), n, g, cap,
+                                       routed ? kSlotDgradDownRouted : kSlotDgradDownShared, s);
+        case kStageDgradGateUp:
+            return launch_grouped_gemm(kMajorK, kMajorMN, kEpiStore, false, calls.begin(), n, g, cap,
+                                       routed ? kSlotDgradGateUpRouted : kSlotDgradGateUpShared, s);
+        default:
+            return launch_grouped_gemm(kMajorMN, kMajorMN, kEpiStore, true, calls.begin(), n, g, cap,
+                                       routed ? kSlotWgradRouted : kSlotWgradShared, s);
+    }
 }
 
 RowMoveParams row_move(const mok_layer_common& c, const PassCtx& x, const Dims& d, int off, int limit, void* local) {
@@ -298,6 +337,8 @@ public:
     Pipeline(const Pipeline&) = delete;
     Pipeline& operator=(const Pipeline&) = delete;
     int error() const { return rc_; }
+    // row movement runs on a side stream beside launches of the caller's stream
+    bool overlaps() const { return use_side_; }
 
     // side stream continues after everything enqueued on main so far / main after side
     int fork() { if (!use_side_) return MOK_OK; forked_ = true; return order(main_, side_); }
@@ -432,17 +473,23 @@ extern "C" int mok_fwd_bf16(const mok_fwd_bf16_args* a, void* stream) {
     MOK_TRY(pipe.error());
     MOK_TRY(pipe.fork());
 
-    // shared expert on the local tokens: its gate|up GEMM runs beside the first dispatch; its down projection beside
-    // the first dispatch too when the window is moved in one piece, beside the last combine chunk when it is chunked
-    MOK_TRY(run_gate_up(c, whole, d, false, 0, d.T, x_local, d.T, a->w_shared_gate, a->w_shared_up, a->gate_shared, a->up_shared,
-                        a->hidden_shared, s));
+    const GemmCall shared_gate_up = gate_up(c, d, false, d.T, x_local, d.T, a->w_shared_gate, a->w_shared_up, a->gate_shared,
+                                            a->up_shared, a->hidden_shared);
+    const GemmCall shared_down = down(c, d, false, d.T, a->hidden_shared, d.T, a->w_shared_down, a->y_shared);
+    // shared expert on the local tokens.  Rows moved in one piece: in the launches of the first window.  Chunked: its
+    // gate|up GEMM runs beside the first dispatch chunk, its down projection beside the last combine chunk.
+    const bool joint = !pipe.overlaps();
     const bool shared_down_last = chunks > 1;
-    if (!shared_down_last) MOK_TRY(run_down(c, whole, d, false, 0, d.T, a->hidden_shared, d.T, a->w_shared_down, a->y_shared, s));
+    if (!joint) {
+        MOK_TRY(launch_stage(kStageGateUp, {shared_gate_up}, c, whole, 0, 0, s));
+        if (!shared_down_last) MOK_TRY(launch_stage(kStageDown, {shared_down}, c, whole, 0, 0, s));
+    }
 
     const int n_macro = (d.cap + d.MB - 1) / d.MB;
     for (int m = n_macro - 1; m >= 0; --m) {
         const int off = m * d.MB;
         const int limit = std::min(d.MB, d.cap - off);
+        const bool with_shared = joint && m == n_macro - 1;
         MOK_TRY(pipe.run(m == 0 || chunk_all_windows(false),
             [&](cudaStream_t st, const PassCtx& x) {
                 RowMoveParams disp = row_move(c, x, d, off, limit, a->x_routed);
@@ -451,9 +498,15 @@ extern "C" int mok_fwd_bf16(const mok_fwd_bf16_args* a, void* stream) {
                 return launch_dispatch_rows(disp, false, move_grid(x), st);
             },
             [&](cudaStream_t st, const PassCtx& x) {
-                MOK_TRY(run_gate_up(c, x, d, true, off, limit, a->x_routed, d.MB, a->w_routed_gate, a->w_routed_up,
-                                    a->gate_routed, a->up_routed, a->hidden_routed, st));
-                return run_down(c, x, d, true, off, limit, a->hidden_routed, d.MB, a->w_routed_down, a->y_routed, st);
+                const GemmCall up = gate_up(c, d, true, limit, a->x_routed, d.MB, a->w_routed_gate, a->w_routed_up,
+                                            a->gate_routed, a->up_routed, a->hidden_routed);
+                const GemmCall dn = down(c, d, true, limit, a->hidden_routed, d.MB, a->w_routed_down, a->y_routed);
+                if (with_shared) {
+                    MOK_TRY(launch_stage(kStageGateUp, {shared_gate_up, up}, c, x, off, limit, st));
+                    return launch_stage(kStageDown, {shared_down, dn}, c, x, off, limit, st);
+                }
+                MOK_TRY(launch_stage(kStageGateUp, {up}, c, x, off, limit, st));
+                return launch_stage(kStageDown, {dn}, c, x, off, limit, st);
             },
             [&](cudaStream_t st, const PassCtx& x) {
                 if (c.defer_combine) return static_cast<int>(MOK_OK);   // mok_fwd_epilogue_rows reads y_routed in place
@@ -461,8 +514,7 @@ extern "C" int mok_fwd_bf16(const mok_fwd_bf16_args* a, void* stream) {
                 comb.peers = combine_peers;
                 return launch_combine_rows(comb, move_grid(x), st);
             }));
-        if (m == 0 && shared_down_last)
-            MOK_TRY(run_down(c, whole, d, false, 0, d.T, a->hidden_shared, d.T, a->w_shared_down, a->y_shared, s));
+        if (m == 0 && shared_down_last) MOK_TRY(launch_stage(kStageDown, {shared_down}, c, whole, 0, 0, s));
         MOK_TRY(pipe.join());      // the next window reuses the buffers
         if (m > 0) MOK_TRY(pipe.fork());
     }
@@ -491,26 +543,33 @@ extern "C" int mok_bwd_bf16(const mok_bwd_bf16_args* a, void* stream) {
     MOK_TRY(pipe.error());
     MOK_TRY(pipe.fork());
 
-    // shared expert (overlaps the first reverse-combine chunk)
-    MOK_TRY(run_dgrad_down(c, whole, d, false, 0, d.T, dy_local, d.T, a->w_shared_down, a->gate_shared, a->up_shared,
-                           a->d_hidden_shared, a->d_gate_shared, a->d_up_shared, nullptr, nullptr, s));
-    MOK_TRY(run_dgrad_gate_up(c, whole, d, false, 0, d.T, a->d_gate_shared, a->d_up_shared, d.T, a->w_shared_gate, a->w_shared_up,
-                              a->d_x_shared, s));
-    MOK_TRY(run_wgrad(c, whole, false, 0, d.T, dy_local, d.H, a->hidden_shared, d.I, d.T, a->d_w_shared_down, 0, s));
-    MOK_TRY(run_wgrad(c, whole, false, 0, d.T, a->d_gate_shared, d.I, x_local, d.H, d.T, a->d_w_shared_gate, 0, s));
-    MOK_TRY(run_wgrad(c, whole, false, 0, d.T, a->d_up_shared, d.I, x_local, d.H, d.T, a->d_w_shared_up, 0, s));
+    const GemmCall sh_dgrad_down = dgrad_down(c, d, false, d.T, dy_local, d.T, a->w_shared_down, a->gate_shared, a->up_shared,
+                                              a->d_hidden_shared, a->d_gate_shared, a->d_up_shared, nullptr, nullptr);
+    const GemmCall sh_dgrad_gate_up = dgrad_gate_up(c, d, false, d.T, a->d_gate_shared, a->d_up_shared, d.T, a->w_shared_gate,
+                                                    a->w_shared_up, a->d_x_shared);
+    const GemmCall sh_wgrad[3] = {wgrad(c, false, dy_local, d.H, a->hidden_shared, d.I, d.T, a->d_w_shared_down, 0),
+                                  wgrad(c, false, a->d_gate_shared, d.I, x_local, d.H, d.T, a->d_w_shared_gate, 0),
+                                  wgrad(c, false, a->d_up_shared, d.I, x_local, d.H, d.T, a->d_w_shared_up, 0)};
+    // shared expert: in the launches of the first window, or ahead of it to overlap the first reverse-combine chunk
+    const bool joint = !pipe.overlaps();
+    if (!joint) {
+        MOK_TRY(launch_stage(kStageDgradDown, {sh_dgrad_down}, c, whole, 0, 0, s));
+        MOK_TRY(launch_stage(kStageDgradGateUp, {sh_dgrad_gate_up}, c, whole, 0, 0, s));
+        MOK_TRY(launch_stage(kStageWgrad, {sh_wgrad[0], sh_wgrad[1], sh_wgrad[2]}, c, whole, 0, 0, s));
+    }
 
     const int n_macro = (d.cap + d.MB - 1) / d.MB;
     for (int m = 0; m < n_macro; ++m) {
         const int off = m * d.MB;
         const int limit = std::min(d.MB, d.cap - off);
+        const bool with_shared = joint && m == 0;
         if (m > 0) {   // replay the forward of this window into the saved-activation buffers
             RowMoveParams disp = row_move(c, whole, d, off, limit, a->x_routed);
             disp.peers = x_peers;
             disp.row_divisor = d.K;
             MOK_TRY(launch_dispatch_rows(disp, false, move_grid(whole), s));
-            MOK_TRY(run_gate_up(c, whole, d, true, off, limit, a->x_routed, d.MB, a->w_routed_gate, a->w_routed_up, a->gate_routed,
-                                a->up_routed, a->hidden_routed, s));
+            MOK_TRY(launch_stage(kStageGateUp, {gate_up(c, d, true, limit, a->x_routed, d.MB, a->w_routed_gate, a->w_routed_up,
+                                                        a->gate_routed, a->up_routed, a->hidden_routed)}, c, whole, off, limit, s));
             MOK_TRY(pipe.fork());
         }
         MOK_TRY(pipe.run(m == 0 || chunk_all_windows(false),
@@ -523,11 +582,17 @@ extern "C" int mok_bwd_bf16(const mok_bwd_bf16_args* a, void* stream) {
                 return launch_dispatch_rows(rc, true, move_grid(x), st);
             },
             [&](cudaStream_t st, const PassCtx& x) {
-                MOK_TRY(run_dgrad_down(c, x, d, true, off, limit, a->d_y_routed, d.MB, a->w_routed_down, a->gate_routed,
-                                       a->up_routed, a->d_hidden_routed, a->d_gate_routed, a->d_up_routed,
-                                       a->router_weights_routed, a->d_router_weight_partials, st));
-                return run_dgrad_gate_up(c, x, d, true, off, limit, a->d_gate_routed, a->d_up_routed, d.MB, a->w_routed_gate,
-                                         a->w_routed_up, a->d_x_routed, st);
+                const GemmCall dd = dgrad_down(c, d, true, limit, a->d_y_routed, d.MB, a->w_routed_down, a->gate_routed,
+                                               a->up_routed, a->d_hidden_routed, a->d_gate_routed, a->d_up_routed,
+                                               a->router_weights_routed, a->d_router_weight_partials);
+                const GemmCall dgu = dgrad_gate_up(c, d, true, limit, a->d_gate_routed, a->d_up_routed, d.MB, a->w_routed_gate,
+                                                   a->w_routed_up, a->d_x_routed);
+                if (with_shared) {
+                    MOK_TRY(launch_stage(kStageDgradDown, {sh_dgrad_down, dd}, c, x, off, limit, st));
+                    return launch_stage(kStageDgradGateUp, {sh_dgrad_gate_up, dgu}, c, x, off, limit, st);
+                }
+                MOK_TRY(launch_stage(kStageDgradDown, {dd}, c, x, off, limit, st));
+                return launch_stage(kStageDgradGateUp, {dgu}, c, x, off, limit, st);
             },
             [&](cudaStream_t st, const PassCtx& x) {
                 RowMoveParams rd = row_move(c, x, d, off, limit, a->d_x_routed);
@@ -542,9 +607,13 @@ extern "C" int mok_bwd_bf16(const mok_bwd_bf16_args* a, void* stream) {
         // point of the caller's stream; the last reverse-dispatch chunk, still running on the side stream, reads
         // d_x_routed and the partials, which they do not touch: they overlap, and the join comes after them
         const int acc = m > 0 ? 1 : 0;
-        MOK_TRY(run_wgrad(c, whole, true, off, limit, a->d_y_routed, d.H, a->hidden_routed, d.I, d.MB, a->d_w_routed_down, acc, s));
-        MOK_TRY(run_wgrad(c, whole, true, off, limit, a->d_gate_routed, d.I, a->x_routed, d.H, d.MB, a->d_w_routed_gate, acc, s));
-        MOK_TRY(run_wgrad(c, whole, true, off, limit, a->d_up_routed, d.I, a->x_routed, d.H, d.MB, a->d_w_routed_up, acc, s));
+        const GemmCall w_down = wgrad(c, true, a->d_y_routed, d.H, a->hidden_routed, d.I, d.MB, a->d_w_routed_down, acc);
+        const GemmCall w_gate = wgrad(c, true, a->d_gate_routed, d.I, a->x_routed, d.H, d.MB, a->d_w_routed_gate, acc);
+        const GemmCall w_up = wgrad(c, true, a->d_up_routed, d.I, a->x_routed, d.H, d.MB, a->d_w_routed_up, acc);
+        if (with_shared)           // the shared expert's tiles contract over all local tokens: the longest go first
+            MOK_TRY(launch_stage(kStageWgrad, {sh_wgrad[0], sh_wgrad[1], sh_wgrad[2], w_down, w_gate, w_up}, c, whole, off, limit, s));
+        else
+            MOK_TRY(launch_stage(kStageWgrad, {w_down, w_gate, w_up}, c, whole, off, limit, s));
         MOK_TRY(pipe.join());      // the next window replays into the buffers the stores read
     }
     return MOK_OK;
@@ -709,10 +778,11 @@ extern "C" int mok_fwd_mxfp8(const mok_fwd_mxfp8_args* a, void* stream) {
     MOK_TRY(pipe.error());
     MOK_TRY(pipe.fork());
 
-    MOK_TRY(run_gate_up(c, whole, d, false, 0, d.T, x_local, d.T, a->w_shared_gate, a->w_shared_up, a->gate_shared, a->up_shared,
-                        a->hidden_shared, s));
+    const GemmCall shared_down = down(c, d, false, d.T, a->hidden_shared, d.T, a->w_shared_down, a->y_shared);
+    MOK_TRY(launch_stage(kStageGateUp, {gate_up(c, d, false, d.T, x_local, d.T, a->w_shared_gate, a->w_shared_up, a->gate_shared,
+                                                a->up_shared, a->hidden_shared)}, c, whole, 0, 0, s));
     const bool shared_down_last = chunks > 1;      // as in mok_fwd_bf16
-    if (!shared_down_last) MOK_TRY(run_down(c, whole, d, false, 0, d.T, a->hidden_shared, d.T, a->w_shared_down, a->y_shared, s));
+    if (!shared_down_last) MOK_TRY(launch_stage(kStageDown, {shared_down}, c, whole, 0, 0, s));
 
     const int n_macro = (d.cap + d.MB - 1) / d.MB;
     for (int m = n_macro - 1; m >= 0; --m) {
@@ -741,8 +811,7 @@ extern "C" int mok_fwd_mxfp8(const mok_fwd_mxfp8_args* a, void* stream) {
                 comb.lean = 1;
                 return launch_combine_rows(comb, move_grid(x), st);
             }));
-        if (m == 0 && shared_down_last)
-            MOK_TRY(run_down(c, whole, d, false, 0, d.T, a->hidden_shared, d.T, a->w_shared_down, a->y_shared, s));
+        if (m == 0 && shared_down_last) MOK_TRY(launch_stage(kStageDown, {shared_down}, c, whole, 0, 0, s));
         MOK_TRY(pipe.join());
         if (m > 0) MOK_TRY(pipe.fork());
     }
@@ -772,13 +841,15 @@ extern "C" int mok_bwd_mxfp8(const mok_bwd_mxfp8_args* a, void* stream) {
     MOK_TRY(pipe.fork());
 
     // shared expert, BF16
-    MOK_TRY(run_dgrad_down(c, whole, d, false, 0, d.T, dy_local, d.T, a->w_shared_down, a->gate_shared, a->up_shared,
-                           a->d_hidden_shared, a->d_gate_shared, a->d_up_shared, nullptr, nullptr, s));
-    MOK_TRY(run_dgrad_gate_up(c, whole, d, false, 0, d.T, a->d_gate_shared, a->d_up_shared, d.T, a->w_shared_gate, a->w_shared_up,
-                              a->d_x_shared, s));
-    MOK_TRY(run_wgrad(c, whole, false, 0, d.T, dy_local, d.H, a->hidden_shared, d.I, d.T, a->d_w_shared_down, 0, s));
-    MOK_TRY(run_wgrad(c, whole, false, 0, d.T, a->d_gate_shared, d.I, x_local, d.H, d.T, a->d_w_shared_gate, 0, s));
-    MOK_TRY(run_wgrad(c, whole, false, 0, d.T, a->d_up_shared, d.I, x_local, d.H, d.T, a->d_w_shared_up, 0, s));
+    MOK_TRY(launch_stage(kStageDgradDown, {dgrad_down(c, d, false, d.T, dy_local, d.T, a->w_shared_down, a->gate_shared, a->up_shared,
+                                                      a->d_hidden_shared, a->d_gate_shared, a->d_up_shared, nullptr, nullptr)},
+                         c, whole, 0, 0, s));
+    MOK_TRY(launch_stage(kStageDgradGateUp, {dgrad_gate_up(c, d, false, d.T, a->d_gate_shared, a->d_up_shared, d.T, a->w_shared_gate,
+                                                           a->w_shared_up, a->d_x_shared)}, c, whole, 0, 0, s));
+    MOK_TRY(launch_stage(kStageWgrad, {wgrad(c, false, dy_local, d.H, a->hidden_shared, d.I, d.T, a->d_w_shared_down, 0),
+                                       wgrad(c, false, a->d_gate_shared, d.I, x_local, d.H, d.T, a->d_w_shared_gate, 0),
+                                       wgrad(c, false, a->d_up_shared, d.I, x_local, d.H, d.T, a->d_w_shared_up, 0)},
+                         c, whole, 0, 0, s));
 
     const int n_macro = (d.cap + d.MB - 1) / d.MB;
     for (int m = 0; m < n_macro; ++m) {
