@@ -615,12 +615,14 @@ def roofline_record(name, wl, res, steps, world):
     T, H, I, E, K = wl["T"], wl["H"], wl["I"], wl["E"], wl["K"]
     peaks = measured_peaks()
     scale = 2.0 if wl.get("mxfp8") else 1.0      # no measured MXFP8 peak on file: twice the measured bf16 figures
-    dom = "gemm_gate_up_swiglu_routed"
-    dom_ms, dom_cnt = res.get("prof", {}).get(dom, (0.0, 0))
+    # on one rank the BF16 launch holds the shared expert's tiles too and is booked under a slot of its own
+    prof = res.get("prof", {})
+    joint = "gemm_gate_up_swiglu_joint" in prof
+    dom = "gemm_gate_up_swiglu_joint" if joint else "gemm_gate_up_swiglu_routed"
+    slots = [prof[k] for k in ("gemm_gate_up_swiglu_joint", "gemm_gate_up_swiglu_routed") if k in prof]
+    dom_ms, dom_cnt = sum(v[0] for v in slots), sum(v[1] for v in slots)
     dom_ms_step = dom_ms / steps if dom_cnt else None
-    # gate + up GEMMs over the T*K routed rows (padding not counted); where the shared expert's tiles are part of the
-    # same launch (one rank, BF16), over its T rows too
-    joint = bool(dom_cnt) and "gemm_gate_up_swiglu_shared" not in res["prof"]
+    # gate + up GEMMs over the T*K routed rows (padding not counted), in a joint launch over the shared expert's T too
     dom_flops = 4.0 * (T * K + (T if joint else 0)) * H * I
     achieved = dom_flops / (dom_ms_step * 1e-3) / 1e12 if dom_ms_step else None
     burst, sustained = scale * peaks["burst"], scale * peaks["tflops"]
@@ -631,7 +633,6 @@ def roofline_record(name, wl, res, steps, world):
                 peak_source=peaks["source"] + (" bf16 figures x2 for fp8" if scale == 2.0 else ""),
                 traffic=dominant_traffic(name, E // world + (1 if joint else 0),
                                          res["n_rows"] + (T if joint else 0) if res.get("n_rows") else None),
-                joint_with_shared_expert=joint,
                 traffic_scope="one step: the launches_per_step launches of this kernel together cover the step's rows "
                               "once and read each local expert's weights once; achieved is over the same launches",
                 launches_per_step=dom_cnt / steps if dom_cnt else 0, ms_per_step=dom_ms_step)

@@ -190,31 +190,31 @@ GemmCall wgrad(const mok_layer_common& c, bool routed, const void* a, int m, con
 enum Stage { kStageGateUp, kStageDown, kStageDgradDown, kStageDgradGateUp, kStageWgrad };
 
 // One launch of a stage.  `calls` may hold shared-expert GEMMs, routed ones, or both (a joint launch, used on one
-// rank where the row movement does not run beside the shared expert).  A launch is booked under the routed slot as
-// soon as it holds routed rows.
+// rank where the row movement does not run beside the shared expert).
 int launch_stage(Stage stage, std::initializer_list<GemmCall> calls, const mok_layer_common& c, const PassCtx& x, int off, int limit,
                  cudaStream_t s) {
-    bool routed = false;
-    for (const GemmCall& k : calls) routed = routed || k.p.routed;
+    bool routed = false, shared = false;
+    for (const GemmCall& k : calls) (k.p.routed ? routed : shared) = true;
     GemmBatch g = gemm_batch(c, x, off, limit);
     if (!routed) g.num_experts = 0;
     const int cap = routed && stage != kStageWgrad ? x.gemm_ctas : 0, n = static_cast<int>(calls.size());
+    auto slot = [&](int of_shared, int of_routed, int of_joint) { return !routed ? of_shared : shared ? of_joint : of_routed; };
     switch (stage) {
         case kStageGateUp:
             return launch_grouped_gemm(kMajorK, kMajorK, kEpiSwigluFwd, false, calls.begin(), n, g, cap,
-                                       routed ? kSlotGateUpRouted : kSlotGateUpShared, s);
+                                       slot(kSlotGateUpShared, kSlotGateUpRouted, kSlotGateUpJoint), s);
         case kStageDown:
             return launch_grouped_gemm(kMajorK, kMajorK, kEpiStore, false, calls.begin(), n, g, cap,
-                                       routed ? kSlotDownRouted : kSlotDownShared, s);
+                                       slot(kSlotDownShared, kSlotDownRouted, kSlotDownJoint), s);
         case kStageDgradDown:
             return launch_grouped_gemm(kMajorK, kMajorMN, kEpiSwigluBwd, false, calls.begin(), n, g, cap,
-                                       routed ? kSlotDgradDownRouted : kSlotDgradDownShared, s);
+                                       slot(kSlotDgradDownShared, kSlotDgradDownRouted, kSlotDgradDownJoint), s);
         case kStageDgradGateUp:
             return launch_grouped_gemm(kMajorK, kMajorMN, kEpiStore, false, calls.begin(), n, g, cap,
-                                       routed ? kSlotDgradGateUpRouted : kSlotDgradGateUpShared, s);
+                                       slot(kSlotDgradGateUpShared, kSlotDgradGateUpRouted, kSlotDgradGateUpJoint), s);
         default:
             return launch_grouped_gemm(kMajorMN, kMajorMN, kEpiStore, true, calls.begin(), n, g, cap,
-                                       routed ? kSlotWgradRouted : kSlotWgradShared, s);
+                                       slot(kSlotWgradShared, kSlotWgradRouted, kSlotWgradJoint), s);
     }
 }
 

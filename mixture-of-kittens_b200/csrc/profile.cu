@@ -58,7 +58,9 @@ extern "C" const char* mok_profile_slot_name(int slot) {
         "gemm_gate_up_swiglu_shared", "gemm_down_shared", "gemm_gate_up_swiglu_routed", "gemm_down_routed",
         "gemm_dgrad_down_swiglu_bwd_shared", "gemm_dgrad_gate_up_shared", "gemm_wgrad_shared",
         "gemm_dgrad_down_swiglu_bwd_routed", "gemm_dgrad_gate_up_routed", "gemm_wgrad_routed",
-        "gemm_plain", "other"};
+        "gemm_plain", "other",
+        "gemm_gate_up_swiglu_joint", "gemm_down_joint", "gemm_dgrad_down_swiglu_bwd_joint", "gemm_dgrad_gate_up_joint",
+        "gemm_wgrad_joint"};
     return (slot >= 0 && slot < mok::kNumSlots) ? names[slot] : "?";
 }
 

@@ -16,6 +16,8 @@ enum ProfSlot : int {
     kSlotDgradDownShared, kSlotDgradGateUpShared, kSlotWgradShared,
     kSlotDgradDownRouted, kSlotDgradGateUpRouted, kSlotWgradRouted,
     kSlotGemmTest, kSlotOther,
+    // launches that hold the shared expert's and the routed GEMMs of a stage
+    kSlotGateUpJoint, kSlotDownJoint, kSlotDgradDownJoint, kSlotDgradGateUpJoint, kSlotWgradJoint,
     kNumSlots
 };
 
