@@ -102,6 +102,13 @@ int mok_schedule(const int32_t* topk_all, int ep_size, int num_local_tokens, int
                  int32_t* num_tokens, int32_t* tokens_per_expert,
                  void* scratch, size_t scratch_bytes, int32_t* status, void* stream);
 
+/* mok_schedule on int64 expert ids (what torch.topk gives), cut to 32 bits as they are read; saves the caller the cast. */
+int mok_schedule_i64(const int64_t* topk_all, int ep_size, int num_local_tokens, int topk,
+                     int num_local_experts, int schedule_capacity, int rank,
+                     int32_t* schedule_peer_rank, int32_t* schedule_peer_token_idx,
+                     int32_t* num_tokens, int32_t* tokens_per_expert,
+                     void* scratch, size_t scratch_bytes, int32_t* status, void* stream);
+
 /* The same scheduler for callers that cannot allocate device memory (a server with a fixed
  * memory plan, a latency-critical loop that must not hit cudaMalloc's device synchronisation, a
  * plug-in host that exposes no allocator): the scratch lives in a fixed 4 MiB __device__ array

@@ -100,10 +100,12 @@ __global__ void __launch_bounds__(256) epilogue_kernel(const uint4* __restrict__
     }
 }
 
-// route -> schedule row, for the epilogues that gather routed rows straight from the GEMM output
+// Route -> schedule row, for the epilogues that gather routed rows straight from the GEMM output.  Entries of routes
+// without a row are left as they are: the reader checks every entry against the schedule itself.
 __global__ void __launch_bounds__(256) invert_rows_kernel(const int* __restrict__ peer_rank, const int* __restrict__ peer_token_idx,
                                                           const int* __restrict__ num_tokens, int row_limit, int routes,
                                                           int* __restrict__ route_row) {
+    pdl_wait();
     const int n = min(*num_tokens, row_limit);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (peer_rank[i] < 0) continue;
@@ -112,57 +114,112 @@ __global__ void __launch_bounds__(256) invert_rows_kernel(const int* __restrict_
     }
 }
 
-// same arithmetic as epilogue_kernel, but the k-th routed row of token t is rows[route_row[t*K+k]]
-// (a route without a row adds nothing); kWeighted = forward, else backward, which also sums each
-// route's router-gradient partials in column order.  `out` may be `shared_rows` itself (the backward pass
-// sums in place: every element is read by the thread that writes it, before it writes), so neither is restrict.
-template <bool kWeighted>
-__global__ void __launch_bounds__(256) epilogue_rows_kernel(const uint4* shared_rows, const uint4* __restrict__ rows,
-                                                            const int* __restrict__ route_row, const float* __restrict__ weights,
-                                                            const float* __restrict__ partials, int partial_cols,
-                                                            float* __restrict__ d_router_weights, uint4* out,
-                                                            int64_t T, int vec_per_row, int K) {
-    const int64_t total = T * vec_per_row;
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
-        const int64_t t = i / vec_per_row;
-        const int v = static_cast<int>(i - t * vec_per_row);
-        const uint4 s = shared_rows[i];
-        float acc[8];
-        {
-            const uint32_t w[4] = {s.x, s.y, s.z, s.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 f = unpack_bf16(w[j]);
-                acc[2 * j] = f.x; acc[2 * j + 1] = f.y;
-            }
-        }
-        for (int k = 0; k < K; ++k) {
-            const int row = route_row[t * K + k];
-            if (!kWeighted && v == 0) {
-                float sum = 0.0f;
-                if (row >= 0)
-                    for (int c = 0; c < partial_cols; ++c) sum += partials[static_cast<size_t>(row) * partial_cols + c];
-                d_router_weights[t * K + k] = sum;
-            }
-            if (row < 0) continue;
-            const uint4 q = rows[static_cast<int64_t>(row) * vec_per_row + v];
-            const float wk = kWeighted ? weights[t * K + k] : 1.0f;
-            const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 f = unpack_bf16(w[j]);
+struct EpilogueRows {
+    const uint4* shared_rows; const uint4* rows; uint4* out;     // out may be shared_rows itself
+    const int* route_row; const int* peer_rank; const int* peer_token_idx; const int* num_tokens;
+    int row_limit;
+    const float* weights;                                        // forward
+    const float* partials; int partial_cols; float* d_router_weights;   // backward
+    int T, vec_per_row, K;
+};
+
+// Same arithmetic as epilogue_kernel, but the k-th routed row of token t is rows[route_row[t*K+k]] (a route without a
+// row adds nothing); kWeighted = forward, else backward, which also sums each route's router-gradient partials in
+// column order.  `out` may be `shared_rows` itself (the backward pass sums in place: every element is read by the
+// thread that writes it, before it writes), so neither is restrict.
+// HBM-bound: (K+2)*H*2 bytes per token.  A block takes a whole token (several where H < 2048), so that a row is read in
+// one piece; while it streams one, it looks up and checks the rows of its next one.
+// Occupancy decides (2048 threads per SM at 32 registers; 1024 threads with four rows in flight each: 160 us).
+// 16384 tokens, H=2048, top-8, with the inversion of the table: 133 us, as with a separate clear and the table walked by
+// every thread (132), 188 with a token cut into 1 KB slices, one per warp.  Where router gradients are summed, by the
+// lookup instead of one thread in 512: H=4096, top-6, forward and backward together 557 -> 472 us.
+constexpr int kEpiThreads = 256, kEpiRoutes = 2;     // routes in flight per thread
+constexpr int kEpiMaxStaged = 1024;                  // routes of one token up to which the table is staged in shared memory
+// tokens per block and step: one load of each thread, and at most 2 x 2048 table entries
+__host__ __device__ constexpr int epi_tokens(int vec_per_row, int K) {
+    const int by_row = kEpiThreads / vec_per_row, by_table = 2048 / K;
+    return by_row <= 1 || by_table <= 1 ? 1 : (by_row < by_table ? by_row : by_table);
+}
+template <bool kWeighted, bool kStaged>
+__global__ void __launch_bounds__(kEpiThreads, 8) epilogue_rows_kernel(const EpilogueRows p) {
+    extern __shared__ int epi_smem[];
+    const int tokens = epi_tokens(p.vec_per_row, p.K), entries = tokens * p.K;
+    int* const s_row = epi_smem;                                            // [2][entries]
+    float* const s_w = reinterpret_cast<float*>(epi_smem + 2 * entries);    // [2][entries]
+    const int groups = (p.T + tokens - 1) / tokens;
+    pdl_wait();
+    const int n_rows = min(*p.num_tokens, p.row_limit);
+
+    auto row_of_route = [&](int route) {
+        const int row = p.route_row[route];
+        return row < 0 || row >= n_rows || p.peer_token_idx[row] != route || p.peer_rank[row] < 0 ? -1 : row;
+    };
+    auto look_up = [&](int group, int buf) {
+        if (kWeighted && !kStaged) return;
+        for (int i = threadIdx.x; i < entries; i += kEpiThreads) {
+            const int route = group * entries + i;
+            int row = -1;
+            if (route < p.T * p.K) {
+                row = row_of_route(route);
                 if (kWeighted) {
-                    acc[2 * j] += __fmul_rn(f.x, wk);
-                    acc[2 * j + 1] += __fmul_rn(f.y, wk);
+                    s_w[buf * entries + i] = p.weights[route];
                 } else {
-                    acc[2 * j] += f.x;
-                    acc[2 * j + 1] += f.y;
+                    float sum = 0.0f;
+                    if (row >= 0) {
+                        const float* part = p.partials + static_cast<size_t>(row) * p.partial_cols;
+#pragma unroll 8
+                        for (int c = 0; c < p.partial_cols; ++c) sum += part[c];
+                    }
+                    p.d_router_weights[route] = sum;
                 }
             }
+            if (kStaged) s_row[buf * entries + i] = row;
         }
-        out[i] = make_uint4(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]), pack_bf16(acc[4], acc[5]),
-                            pack_bf16(acc[6], acc[7]));
+    };
+
+    int buf = 0;
+    if (blockIdx.x < groups) look_up(blockIdx.x, 0);
+    for (int g = blockIdx.x; g < groups; g += gridDim.x, buf ^= 1) {
+        __syncthreads();                             // this group's rows are in; the other buffer is no longer read
+        if (g + static_cast<int>(gridDim.x) < groups) look_up(g + gridDim.x, buf ^ 1);
+        for (int i = threadIdx.x; i < tokens * p.vec_per_row; i += kEpiThreads) {
+            const int sub = tokens > 1 ? i / p.vec_per_row : 0, v = i - sub * p.vec_per_row;
+            if (g * tokens + sub >= p.T) break;
+            const long long at = static_cast<long long>(g * tokens + sub) * p.vec_per_row + v;
+            const int* row_of = s_row + buf * entries + sub * p.K;
+            const float* w_of = s_w + buf * entries + sub * p.K;
+            const int route0 = (g * tokens + sub) * p.K;
+            float acc[8];
+            {
+                const uint4 s = p.shared_rows[at];
+                const uint32_t w[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { const float2 f = unpack_bf16(w[j]); acc[2 * j] = f.x; acc[2 * j + 1] = f.y; }
+            }
+            for (int k = 0; k < p.K; k += kEpiRoutes) {
+                int row[kEpiRoutes];
+                uint4 q[kEpiRoutes];
+#pragma unroll
+                for (int r = 0; r < kEpiRoutes; ++r) {
+                    row[r] = k + r < p.K ? (kStaged ? row_of[k + r] : row_of_route(route0 + k + r)) : -1;
+                    q[r] = row[r] >= 0 ? p.rows[static_cast<long long>(row[r]) * p.vec_per_row + v] : make_uint4(0, 0, 0, 0);
+                }
+#pragma unroll
+                for (int r = 0; r < kEpiRoutes; ++r) {
+                    if (row[r] < 0) continue;
+                    const float wk = kWeighted ? (kStaged ? w_of[k + r] : p.weights[route0 + k + r]) : 1.0f;
+                    const uint32_t w[4] = {q[r].x, q[r].y, q[r].z, q[r].w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 f = unpack_bf16(w[j]);
+                        acc[2 * j] += kWeighted ? __fmul_rn(f.x, wk) : f.x;
+                        acc[2 * j + 1] += kWeighted ? __fmul_rn(f.y, wk) : f.y;
+                    }
+                }
+            }
+            p.out[at] = make_uint4(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]), pack_bf16(acc[4], acc[5]),
+                                   pack_bf16(acc[6], acc[7]));
+        }
     }
 }
 
@@ -211,6 +268,7 @@ __global__ void __launch_bounds__(kMoveMaxWarps * 32, 8) move_rows_kernel(RowMov
         mbar_fence_init();
     }
     __syncthreads();
+    pdl_wait();
 
     const int n_total = min(*p.num_tokens, p.capacity);
     const int win_rows = max(0, min(n_total - p.row_offset, p.row_limit));
@@ -328,6 +386,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) dispatch_quant_kern
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) { abort_word = 0; mbar_init(&bars[0], 1); mbar_init(&bars[1], 1); mbar_fence_init(); }
     __syncthreads();
+    pdl_wait();
 
     const int n_total = min(*p.num_tokens, p.capacity);
     const int win_rows = max(0, min(n_total - p.row_offset, p.row_limit));
@@ -412,14 +471,11 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) dispatch_quant_kern
 int launch_dispatch_quant(const RowMoveParams& p, const QuantOut& out, bool scale, int num_blocks, cudaStream_t stream) {
     ProfScope prof(kSlotDispatch, stream);
     if (p.lean) {
-        if (scale) dispatch_quant_kernel<true, 64, 128><<<num_blocks, 64, 0, stream>>>(p, out);
-        else dispatch_quant_kernel<false, 64, 128><<<num_blocks, 64, 0, stream>>>(p, out);
-    } else {
-        if (scale) dispatch_quant_kernel<true, 256, 256><<<num_blocks, 256, 0, stream>>>(p, out);
-        else dispatch_quant_kernel<false, 256, 256><<<num_blocks, 256, 0, stream>>>(p, out);
+        auto* kern = scale ? dispatch_quant_kernel<true, 64, 128> : dispatch_quant_kernel<false, 64, 128>;
+        return launch_kernel(kern, num_blocks, 64, 0, stream, false, p.dependent != 0, p, out);
     }
-    MOK_CUDA_CHECK(cudaGetLastError());
-    return MOK_OK;
+    auto* kern = scale ? dispatch_quant_kernel<true, 256, 256> : dispatch_quant_kernel<false, 256, 256>;
+    return launch_kernel(kern, num_blocks, 256, 0, stream, false, p.dependent != 0, p, out);
 }
 
 // Three shapes of mover CTA: "thin" (3 warps x 2 x 4 KB = 24 KB, many CTAs, fits beside a BF16 GEMM CTA), "lean"
@@ -438,9 +494,7 @@ int launch_move(RowMoveParams p, int num_blocks, cudaStream_t stream) {
         MOK_CUDA_CHECK(cudaFuncSetAttribute(move_rows_kernel<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 2 * 8192));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    move_rows_kernel<kMode><<<num_blocks, warps * 32, smem, stream>>>(p);
-    MOK_CUDA_CHECK(cudaGetLastError());
-    return MOK_OK;
+    return launch_kernel(move_rows_kernel<kMode>, num_blocks, warps * 32, smem, stream, false, p.dependent != 0, p);
 }
 
 int launch_dispatch_rows(const RowMoveParams& p, bool scale, int num_blocks, cudaStream_t stream) {
@@ -534,13 +588,16 @@ extern "C" int mok_bwd_epilogue(const void* d_x_shared, const void* d_x_routed_b
 }
 
 namespace {
-int invert_rows(const int32_t* peer_rank, const int32_t* peer_token_idx, const int32_t* num_tokens, int32_t* route_row,
-                int routes, int row_limit, cudaStream_t s) {
-    MOK_CUDA_CHECK(cudaMemsetAsync(route_row, 0xFF, static_cast<size_t>(routes) * sizeof(int32_t), s));
-    mok::invert_rows_kernel<<<std::min(1024, (row_limit + 255) / 256), 256, 0, s>>>(peer_rank, peer_token_idx, num_tokens, row_limit,
-                                                                                    routes, route_row);
-    MOK_CUDA_CHECK(cudaGetLastError());
-    return MOK_OK;
+int epilogue_rows(bool weighted, const mok::EpilogueRows& p, int32_t* route_row, cudaStream_t s) {
+    ProfScope prof(kSlotEpilogue, s, 2);
+    MOK_TRY(launch_kernel(mok::invert_rows_kernel, std::min(1024, (p.row_limit + 255) / 256), 256, 0, s, false, true, p.peer_rank,
+                          p.peer_token_idx, p.num_tokens, p.row_limit, p.T * p.K, route_row));
+    const int tokens = epi_tokens(p.vec_per_row, p.K), groups = (p.T + tokens - 1) / tokens;
+    const bool staged = p.K <= kEpiMaxStaged;
+    const size_t smem = staged ? static_cast<size_t>(2) * tokens * p.K * 8 : 0;
+    auto* kern = weighted ? (staged ? mok::epilogue_rows_kernel<true, true> : mok::epilogue_rows_kernel<true, false>)
+                          : (staged ? mok::epilogue_rows_kernel<false, true> : mok::epilogue_rows_kernel<false, false>);
+    return launch_kernel(kern, std::min(groups, 16 * device_sm_count()), kEpiThreads, smem, s, false, true, p);
 }
 }  // namespace
 
@@ -553,15 +610,16 @@ extern "C" int mok_fwd_epilogue_rows(const void* y_shared, const void* y_routed,
         return MOK_ERR_INVALID;
     if (num_local_tokens <= 0 || hidden <= 0 || hidden % 8 || topk <= 0 || row_limit <= 0) return MOK_ERR_INVALID;
     if (static_cast<int64_t>(num_local_tokens) * topk > INT32_MAX) return MOK_ERR_TOO_LARGE;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int vpr = hidden / 8;
-    ProfScope prof(kSlotEpilogue, s, 2);
-    MOK_TRY(invert_rows(schedule_peer_rank, schedule_peer_token_idx, num_tokens, route_row, num_local_tokens * topk, row_limit, s));
-    mok::epilogue_rows_kernel<true><<<epilogue_grid(static_cast<int64_t>(num_local_tokens) * vpr), 256, 0, s>>>(
-        static_cast<const uint4*>(y_shared), static_cast<const uint4*>(y_routed), route_row, topk_weights, nullptr, 0, nullptr,
-        static_cast<uint4*>(output), num_local_tokens, vpr, topk);
-    MOK_CUDA_CHECK(cudaGetLastError());
-    return MOK_OK;
+    mok::EpilogueRows p{};
+    p.shared_rows = static_cast<const uint4*>(y_shared);
+    p.rows = static_cast<const uint4*>(y_routed);
+    p.out = static_cast<uint4*>(output);
+    p.route_row = route_row;
+    p.peer_rank = schedule_peer_rank; p.peer_token_idx = schedule_peer_token_idx; p.num_tokens = num_tokens;
+    p.row_limit = row_limit;
+    p.weights = topk_weights;
+    p.T = num_local_tokens; p.vec_per_row = hidden / 8; p.K = topk;
+    return epilogue_rows(true, p, route_row, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int mok_bwd_epilogue_rows(const void* d_x_shared, const void* d_x_routed, const float* partials, int partial_cols,
@@ -574,13 +632,14 @@ extern "C" int mok_bwd_epilogue_rows(const void* d_x_shared, const void* d_x_rou
     if (num_local_tokens <= 0 || hidden <= 0 || hidden % 8 || topk <= 0 || row_limit <= 0 || partial_cols <= 0)
         return MOK_ERR_INVALID;
     if (static_cast<int64_t>(num_local_tokens) * topk > INT32_MAX) return MOK_ERR_TOO_LARGE;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int vpr = hidden / 8;
-    ProfScope prof(kSlotEpilogue, s, 2);
-    MOK_TRY(invert_rows(schedule_peer_rank, schedule_peer_token_idx, num_tokens, route_row, num_local_tokens * topk, row_limit, s));
-    mok::epilogue_rows_kernel<false><<<epilogue_grid(static_cast<int64_t>(num_local_tokens) * vpr), 256, 0, s>>>(
-        static_cast<const uint4*>(d_x_shared), static_cast<const uint4*>(d_x_routed), route_row, nullptr, partials, partial_cols,
-        d_router_weights, static_cast<uint4*>(d_x), num_local_tokens, vpr, topk);
-    MOK_CUDA_CHECK(cudaGetLastError());
-    return MOK_OK;
+    mok::EpilogueRows p{};
+    p.shared_rows = static_cast<const uint4*>(d_x_shared);
+    p.rows = static_cast<const uint4*>(d_x_routed);
+    p.out = static_cast<uint4*>(d_x);
+    p.route_row = route_row;
+    p.peer_rank = schedule_peer_rank; p.peer_token_idx = schedule_peer_token_idx; p.num_tokens = num_tokens;
+    p.row_limit = row_limit;
+    p.partials = partials; p.partial_cols = partial_cols; p.d_router_weights = d_router_weights;
+    p.T = num_local_tokens; p.vec_per_row = hidden / 8; p.K = topk;
+    return epilogue_rows(false, p, route_row, static_cast<cudaStream_t>(stream));
 }

@@ -40,6 +40,20 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 }
 
 // ---------------------------------------------------------------------------------------
+// Programmatic dependent launch.  Every kernel of the library calls pdl_wait() before it touches global memory: it
+// returns once the kernels ahead of it on the stream have finished and their writes are visible (at once without the
+// launch attribute).  From then on the next kernel's CTAs may be placed and run their prologue while this one runs and
+// drains.  Only shared memory, tensor memory and kernel parameters may be touched before it.
+// The next kernel is let in after the wait, not at entry: let in at entry, a chain of short kernels piles up on the
+// SMs and the one that runs gets the slots the waiting ones left (scheduler of eight ranks, back to back: 29.5 us so,
+// 18.8 us with one kernel ahead at most).
+// ---------------------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// ---------------------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -316,5 +330,32 @@ void note_error_text(const char* text);
             return MOK_ERR_CUDA;                                   \
         }                                                          \
     } while (0)
+
+// Launch with optional clusters of two CTAs and optional programmatic dependence on the kernel ahead (see pdl_wait).
+template <class... Params, class... Args>
+int launch_kernel(void (*kern)(Params...), int grid, int threads, size_t smem, cudaStream_t stream, bool pairs, bool dependent,
+                  const Args&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(pairs ? grid & ~1 : grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2] = {};
+    int n = 0;
+    if (pairs) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = 2; attr[n].val.clusterDim.y = 1; attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    if (dependent) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    MOK_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...));
+    return MOK_OK;
+}
 
 }  // namespace mok

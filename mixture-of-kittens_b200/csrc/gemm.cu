@@ -77,23 +77,7 @@ int launch_inst(const GemmBatch& batch, int grid, cudaStream_t stream) {
         MOK_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemBytes));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    if (k2) {      // pairs of CTAs on neighbouring SMs: cluster of 2
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(grid & ~1);
-        cfg.blockDim = dim3(kGemmThreads);
-        cfg.dynamicSmemBytes = kGemmSmemBytes;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        MOK_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, batch));
-    } else {
-        kern<<<grid, kGemmThreads, kGemmSmemBytes, stream>>>(batch);
-    }
-    MOK_CUDA_CHECK(cudaGetLastError());
-    return MOK_OK;
+    return launch_kernel(kern, grid, kGemmThreads, kGemmSmemBytes, stream, k2, batch.dependent != 0, batch);
 }
 
 }  // namespace

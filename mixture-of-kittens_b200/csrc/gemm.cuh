@@ -87,6 +87,7 @@ struct GemmBatch {
     float limit;
     int has_limit;
     int* status;
+    int dependent;                 // host side: launch with programmatic dependence on the kernel ahead
 };
 
 // sigmoid through one tanh.approx (a single special-function op instead of exp + reciprocal):
@@ -137,6 +138,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmBatch g) {
         if (k2) { tmem_alloc_pair(tmem_slot, kTmemCols); tmem_relinquish_pair(); }
         else { tmem_alloc(tmem_slot, kTmemCols); tmem_relinquish(); }
     }
+    pdl_wait();
     if (warp == 0 && E > 0) {      // inclusive prefix of padded rows per expert
 #pragma unroll 8
         for (int e = lane; e < E; e += 32) s_end[e] = g.tokens_per_expert[e];

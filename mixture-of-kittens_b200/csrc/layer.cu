@@ -56,6 +56,7 @@ struct PassCtx {
     ChunkSpec chunk = {0, 1, 0};   // row sub-range of the window the launch covers
     int gemm_ctas = 0;             // cap on the CTAs of routed GEMM launches (0 = all SMs)
     int comm_sms = 0;              // > 0: the call's communication-SM budget applies to the row movers of this launch
+    bool dependent = false;        // launches depend programmatically on the kernel ahead of them on the stream
     bool dedicated = false;        // the budget is SMs of the movers' own (fat CTAs), not mover CTAs beside the GEMM CTAs
 };
 
@@ -72,6 +73,7 @@ GemmBatch gemm_batch(const mok_layer_common& c, const PassCtx& x, int off, int l
     g.limit = c.swiglu_limit;
     g.has_limit = c.has_swiglu_limit;
     g.status = c.status;
+    g.dependent = x.dependent ? 1 : 0;
     return g;
 }
 
@@ -232,6 +234,7 @@ RowMoveParams row_move(const mok_layer_common& c, const PassCtx& x, const Dims& 
     r.status = c.status;
     r.fat_ctas = (x.comm_sms > 0 && x.dedicated) ? 1 : 0;
     r.chunk = x.chunk;
+    r.dependent = x.dependent ? 1 : 0;
     return r;
 }
 
@@ -339,6 +342,9 @@ public:
     int error() const { return rc_; }
     // row movement runs on a side stream beside launches of the caller's stream
     bool overlaps() const { return use_side_; }
+    // Programmatic dependence only where all launches of the pass are on one stream: with row movement on a side stream,
+    // a GEMM CTA that is placed early would hold an SM that mover CTAs could use.
+    PassCtx whole() const { PassCtx x; x.dependent = !use_side_; return x; }
 
     // side stream continues after everything enqueued on main so far / main after side
     int fork() { if (!use_side_) return MOK_OK; forked_ = true; return order(main_, side_); }
@@ -350,7 +356,7 @@ public:
         if (rc_ != MOK_OK) return rc_;
         int rc = MOK_OK;
         if (chunks_ <= 1 || !chunked) {
-            PassCtx x;
+            const PassCtx x = whole();
             if (use_side_ && forked_) {
                 if ((rc = load(side_, x))) return rc;
                 if ((rc = join())) return rc;
@@ -469,7 +475,7 @@ extern "C" int mok_fwd_bf16(const mok_fwd_bf16_args* a, void* stream) {
     const void* x_local = x_peers.p[d.rank];
     const int chunks = pipeline_chunks(c, std::min(d.MB, d.cap));
     Pipeline pipe(s, chunks, c.minibatch_size, pipeline_comm_sms(c, chunks));
-    const PassCtx whole;       // launches outside the chunked pipeline cover their whole window on all SMs
+    const PassCtx whole = pipe.whole();    // launches outside the chunked pipeline cover their whole window on all SMs
     MOK_TRY(pipe.error());
     MOK_TRY(pipe.fork());
 
@@ -539,7 +545,7 @@ extern "C" int mok_bwd_bf16(const mok_bwd_bf16_args* a, void* stream) {
     const int partial_cols = d.I / kBlockN * kEpiSplit;
     const int chunks = pipeline_chunks(c, std::min(d.MB, d.cap));
     Pipeline pipe(s, chunks, c.minibatch_size, pipeline_comm_sms(c, chunks));
-    const PassCtx whole;       // launches outside the chunked pipeline cover their whole window on all SMs
+    const PassCtx whole = pipe.whole();    // launches outside the chunked pipeline cover their whole window on all SMs
     MOK_TRY(pipe.error());
     MOK_TRY(pipe.fork());
 
@@ -699,6 +705,7 @@ MxGemmParams mx_base(const mok_layer_common& c, const PassCtx& x, int off, int l
     p.status = c.status;
     p.q_cols = c.intermediate;
     p.t_rows = c.macrobatch_size;
+    p.dependent = x.dependent ? 1 : 0;
     return p;
 }
 inline uint8_t* u8(void* p) { return static_cast<uint8_t*>(p); }
@@ -774,7 +781,7 @@ extern "C" int mok_fwd_mxfp8(const mok_fwd_mxfp8_args* a, void* stream) {
     const void* x_local = x_peers.p[d.rank];
     const int chunks = pipeline_chunks(c, std::min(d.MB, d.cap));
     Pipeline pipe(s, chunks, c.minibatch_size, pipeline_comm_sms(c, chunks));
-    const PassCtx whole;       // launches outside the chunked pipeline cover their whole window on all SMs
+    const PassCtx whole = pipe.whole();    // launches outside the chunked pipeline cover their whole window on all SMs
     MOK_TRY(pipe.error());
     MOK_TRY(pipe.fork());
 
@@ -836,7 +843,7 @@ extern "C" int mok_bwd_mxfp8(const mok_bwd_mxfp8_args* a, void* stream) {
     const int partial_cols = d.I / kBlockN;
     const int chunks = pipeline_chunks(c, std::min(d.MB, d.cap));
     Pipeline pipe(s, chunks, c.minibatch_size, pipeline_comm_sms(c, chunks));
-    const PassCtx whole;       // launches outside the chunked pipeline cover their whole window on all SMs
+    const PassCtx whole = pipe.whole();    // launches outside the chunked pipeline cover their whole window on all SMs
     MOK_TRY(pipe.error());
     MOK_TRY(pipe.fork());
 

@@ -25,23 +25,7 @@ int launch_mx_inst(const CUtensorMap& a0, const CUtensorMap& b0, const CUtensorM
         MOK_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    if (k2) {      // pairs of CTAs on neighbouring SMs: cluster of 2
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(grid & ~1);
-        cfg.blockDim = dim3(kMxThreads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        MOK_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, a0, b0, a1, b1, sf, p));
-    } else {
-        kern<<<grid, kMxThreads, smem, stream>>>(a0, b0, a1, b1, sf, p);
-    }
-    MOK_CUDA_CHECK(cudaGetLastError());
-    return MOK_OK;
+    return launch_kernel(kern, grid, kMxThreads, smem, stream, k2, p.dependent != 0, a0, b0, a1, b1, sf, p);
 }
 
 // two-CTA tiles unless MOK_B200_MX_2CTA=0 (or MOK_B200_2CTA=0, which switches both GEMM families)

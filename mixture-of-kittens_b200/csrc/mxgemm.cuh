@@ -96,6 +96,7 @@ struct MxGemmParams {
     float limit;
     int has_limit;
     int* status;
+    int dependent;                          // host side: launch with programmatic dependence on the kernel ahead
 };
 
 struct MxScaleMaps {               // unswizzled tensor maps over [tiles, 512 B] scale arrays
@@ -168,9 +169,6 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int E = p.tokens_per_expert ? p.num_experts : 1;
-    if (p.tokens_per_expert) {
-        for (int e = threadIdx.x; e < E; e += blockDim.x) s_end[e] = p.tokens_per_expert[e];
-    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < kMxStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
         mbar_init(tfull_bar, 1);
@@ -178,8 +176,15 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
         *abort_flag = 0;
         mbar_fence_init();
     }
-    __syncthreads();
+    if (warp == 1) {
+        if (k2) { tmem_alloc_pair(tmem_slot, kTmemCols); tmem_relinquish_pair(); }
+        else { tmem_alloc(tmem_slot, kTmemCols); tmem_relinquish(); }
+    }
+    pdl_wait();
     if (warp == 0 && p.tokens_per_expert) {
+#pragma unroll 8
+        for (int e = lane; e < E; e += 32) s_end[e] = p.tokens_per_expert[e];
+        __syncwarp();
         const int per = (E + 31) / 32;
         int sum = 0;
         for (int j = 0; j < per; ++j) { const int e = lane * per + j; if (e < E) sum += s_end[e]; }
@@ -188,10 +193,6 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
         for (int off = 1; off < 32; off <<= 1) { const int n = __shfl_up_sync(0xffffffffu, incl, off); if (lane >= off) incl += n; }
         int run = incl - sum;
         for (int j = 0; j < per; ++j) { const int e = lane * per + j; if (e < E) { run += s_end[e]; s_end[e] = run; } }
-    }
-    if (warp == 1) {
-        if (k2) { tmem_alloc_pair(tmem_slot, kTmemCols); tmem_relinquish_pair(); }
-        else { tmem_alloc(tmem_slot, kTmemCols); tmem_relinquish(); }
     }
     tc_fence_before();
     __syncthreads();

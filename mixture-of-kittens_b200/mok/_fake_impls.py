@@ -31,6 +31,13 @@ def _(barrier_buffer, barrier_buffer_ptrs, barrier_buffer_multicast_ptr, target)
     return None
 
 
+@_fake("mok::schedule_local")
+def _(top_experts, num_local_experts, schedule_capacity):
+    i32 = torch.int32
+    return (_new(top_experts, (schedule_capacity,), i32), _new(top_experts, (schedule_capacity,), i32),
+            _new(top_experts, (1,), i32), _new(top_experts, (num_local_experts,), i32))
+
+
 @_fake("mok::schedule")
 def _(topk_all, num_local_experts, schedule_capacity, rank):
     i32 = torch.int32

@@ -125,6 +125,8 @@ mok_barrier_all = _sig("mok_barrier_all", C.c_int, [vp, u64p, C.c_int, vp, vp, C
 mok_schedule_scratch_bytes = _sig("mok_schedule_scratch_bytes", C.c_size_t, [C.c_int, C.c_int])
 mok_schedule = _sig("mok_schedule", C.c_int, [vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int,
                                               vp, vp, vp, vp, vp, C.c_size_t, vp, vp])
+mok_schedule_i64 = _sig("mok_schedule_i64", C.c_int, [vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int,
+                                                      vp, vp, vp, vp, vp, C.c_size_t, vp, vp])
 mok_schedule_static_max_scratch_bytes = _sig("mok_schedule_static_max_scratch_bytes", C.c_size_t, [])
 mok_schedule_static = _sig("mok_schedule_static", C.c_int, [vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int,
                                                             vp, vp, vp, vp, vp, vp])

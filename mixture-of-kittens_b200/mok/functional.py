@@ -299,16 +299,16 @@ def build_schedule(workspace: MoKWorkspace, config: MoKConfig, top_experts: torc
     if type(num_local_experts) is not int or num_local_experts <= 0:
         raise ValueError("num_local_experts must be a positive integer")
 
-    if workspace.ep_size == 1 and SINGLE_RANK_FAST_PATH:           # nothing to gather: the scheduler reads the routes where the cast put them
-        topk_all = top_experts.to(torch.int32).unsqueeze(0)
+    if workspace.ep_size == 1 and SINGLE_RANK_FAST_PATH:           # nothing to gather: the scheduler reads the caller's routes
+        peer_rank, peer_token_idx, num_tokens, tokens_per_expert = ops.schedule_local(
+            top_experts, num_local_experts, workspace.schedule_capacity)
     else:
         ops.all_gather_top_experts(top_experts.to(torch.int32), workspace.all_gather_top_experts_buffer,
                                    workspace.all_gather_top_experts_buffer_multicast_ptr, workspace.ep_rank,
                                    config.all_gather_top_experts_chunk_bytes)
         _barrier(workspace)
-        topk_all = workspace.all_gather_top_experts_buffer
-    peer_rank, peer_token_idx, num_tokens, tokens_per_expert = ops.schedule(
-        topk_all, num_local_experts, workspace.schedule_capacity, workspace.ep_rank)
+        peer_rank, peer_token_idx, num_tokens, tokens_per_expert = ops.schedule(
+            workspace.all_gather_top_experts_buffer, num_local_experts, workspace.schedule_capacity, workspace.ep_rank)
     return MoKSchedule(peer_rank=peer_rank, peer_token_idx=peer_token_idx, num_tokens=num_tokens,
                        tokens_per_expert=tokens_per_expert)
 

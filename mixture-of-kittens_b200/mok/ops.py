@@ -283,6 +283,11 @@ def schedule(topk_all: Tensor, num_local_experts: int, schedule_capacity: int,
     _need(num_local_experts <= _lib.MAX_LOCAL_EXPERTS, "num_local_experts exceeds this build's limit of 1024",
           NotImplementedError)
 
+    return _run_schedule(_lib.mok_schedule, topk_all, num_local_experts, schedule_capacity, rank)
+
+
+def _run_schedule(entry, topk_all: Tensor, num_local_experts: int, schedule_capacity: int, rank: int):
+    ep_size, tokens, topk = topk_all.shape
     dev = topk_all.device
     i32 = dict(dtype=torch.int32, device=dev)
     peer_rank = torch.empty(schedule_capacity, **i32)
@@ -291,11 +296,30 @@ def schedule(topk_all: Tensor, num_local_experts: int, schedule_capacity: int,
     tokens_per_expert = torch.empty(num_local_experts, **i32)
     scratch_bytes = _lib.mok_schedule_scratch_bytes(ep_size, num_local_experts)
     scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=dev)
-    _lib.check(_lib.mok_schedule(topk_all.data_ptr(), ep_size, tokens, topk, num_local_experts, schedule_capacity, rank,
-                                 peer_rank.data_ptr(), peer_tok.data_ptr(), num_tokens.data_ptr(),
-                                 tokens_per_expert.data_ptr(), scratch.data_ptr(), scratch_bytes,
-                                 _lib.status_tensor(dev).data_ptr(), _lib.stream_ptr(dev)), "schedule")
+    _lib.check(entry(topk_all.data_ptr(), ep_size, tokens, topk, num_local_experts, schedule_capacity, rank,
+                     peer_rank.data_ptr(), peer_tok.data_ptr(), num_tokens.data_ptr(),
+                     tokens_per_expert.data_ptr(), scratch.data_ptr(), scratch_bytes,
+                     _lib.status_tensor(dev).data_ptr(), _lib.stream_ptr(dev)), "schedule")
     return peer_rank, peer_tok, num_tokens, tokens_per_expert
+
+
+@_operator("mok::schedule_local", mutates_args=())
+def schedule_local(top_experts: Tensor, num_local_experts: int, schedule_capacity: int) -> tuple[Tensor, Tensor, Tensor, Tensor]:
+    """`schedule` of a single rank straight from the int64 routes [num_local_tokens, topk] a router gives: nothing is
+    gathered and nothing cast in between.  No reference counterpart (the reference casts to int32, mok/functional.py:380-384)."""
+    _need(top_experts.ndim == 2, "top_experts must have shape (num_local_tokens, topk)")
+    tokens, topk = top_experts.shape
+    _need(tokens >= 512 and tokens % 256 == 0, "top_experts num_local_tokens must be at least 512 and divisible by 256")
+    _need(0 < topk <= 255, "top_experts topk must be in [1, 255]")
+    _need(type(num_local_experts) is int and num_local_experts > 0, "num_local_experts must be a positive integer")
+    _need(type(schedule_capacity) is int and schedule_capacity > 0 and schedule_capacity % 256 == 0,
+          "schedule_capacity must be positive and divisible by 256")
+    _need(schedule_capacity >= tokens * topk, "schedule_capacity must hold at least one rank's routed tokens")
+    _need(top_experts.is_cuda and top_experts.dtype == torch.int64 and top_experts.is_contiguous(),
+          "top_experts must be a contiguous CUDA int64 tensor", TypeError)
+    _need(num_local_experts <= _lib.MAX_LOCAL_EXPERTS, "num_local_experts exceeds this build's limit of 1024",
+          NotImplementedError)
+    return _run_schedule(_lib.mok_schedule_i64, top_experts.unsqueeze(0), num_local_experts, schedule_capacity, 0)
 
 
 # ------------------------------------------------------------------------------------------

@@ -81,6 +81,78 @@ def test_schedule_overflow_sets_status_not_trap(cuda_device):
     assert np.array_equal(ref[0], pr.cpu().numpy())   # in-range slots are still exact
 
 
+@pytest.mark.parametrize("W,T,K,El,skip", [(1, 512, 8, 512, 0),      # the most experts whose offsets the place kernel finds itself
+                                           (1, 512, 8, 513, 0), (4, 512, 3, 129, 0),     # just beyond, with the scan kernel
+                                           (8, 512, 2, 64, 1),                           # routes on a 4- / 8-byte boundary only
+                                           (1, 513, 3, 5, 0), (2, 331, 1, 2, 0), (3, 1, 1, 1, 0)])   # odd route counts
+def test_schedule_int32_and_int64_ids_and_alignment(cuda_device, W, T, K, El, skip):
+    """Both widths of expert ids, both ways of finding offsets, aligned and unaligned tables: all equal to the oracle."""
+    L = _mok()._lib
+    g = torch.Generator().manual_seed(T + El)
+    topk = torch.topk(torch.randn(W, T, max(W * El, K), generator=g), K, dim=2).indices
+    cap = T * K * W + El * 256 + (3 if T % 256 else 0)
+    scratch = torch.empty(L.mok_schedule_scratch_bytes(W, El), dtype=torch.uint8, device=cuda_device)
+    for rank in sorted({0, W - 1}):
+        ref = O.schedule_tables(topk.numpy().astype(np.int32), El, cap, rank)
+        for dtype, entry in ((torch.int32, L.mok_schedule), (torch.int64, L.mok_schedule_i64)):
+            flat = torch.zeros(topk.numel() + skip, dtype=dtype, device=cuda_device)
+            flat[skip:] = topk.reshape(-1).to(dtype)
+            if dtype == torch.int64:
+                flat[skip:] += (torch.arange(topk.numel(), device=cuda_device) % 2) << 40     # cut off by the 32-bit read
+            tables = torch.full((2 * (cap + skip),), 7, dtype=torch.int32, device=cuda_device)
+            pr, pt = tables[skip:skip + cap], tables[cap + 2 * skip:]
+            nt, tpe = torch.zeros(1, dtype=torch.int32, device=cuda_device), torch.zeros(El, dtype=torch.int32, device=cuda_device)
+            L.check(entry(flat.data_ptr() + skip * flat.element_size(), W, T, K, El, cap, rank, pr.data_ptr(), pt.data_ptr(),
+                          nt.data_ptr(), tpe.data_ptr(), scratch.data_ptr(), scratch.numel(),
+                          L.status_tensor(cuda_device).data_ptr(), L.stream_ptr(cuda_device)), "schedule")
+            torch.cuda.synchronize()
+            for r, t in zip(ref, (pr, pt, nt, tpe)):
+                assert np.array_equal(r, t.cpu().numpy()), (dtype, rank)
+
+
+@pytest.mark.parametrize("T,H,K", [(512, 256, 2), (768, 1280, 33), (512, 2304, 5), (3, 8, 300), (5, 24, 1025)])
+def test_epilogue_rows_checks_every_route_entry(cuda_device, T, H, K):
+    """The route table is not cleared before it is filled: whatever an entry of a route without a row holds (another
+    row, a padding row, anything out of range), the route adds nothing.  Sums are in k order, so the result is exact."""
+    L = _mok()._lib
+    g = torch.Generator(device=cuda_device).manual_seed(K)
+    rows = T * K // 2 + 512                                     # half of the routes have a row
+    perm = torch.randperm(T * K, generator=g, device=cuda_device)
+    tok = torch.full((rows,), -1, dtype=torch.int32, device=cuda_device)
+    live = torch.randperm(rows - 256, generator=g, device=cuda_device)[:T * K // 2]
+    tok[live] = perm[:T * K // 2].int()
+    rank = torch.where(tok >= 0, 0, -1).int()
+    n = torch.tensor([rows - 256], dtype=torch.int32, device=cuda_device)
+    shared = torch.randn(T, H, generator=g, device=cuda_device).bfloat16()
+    y = torch.randn(rows, H, generator=g, device=cuda_device).bfloat16()
+    w = torch.rand(T, K, generator=g, device=cuda_device)
+    parts = torch.randn(rows, 6, generator=g, device=cuda_device)
+    row_of = torch.full((T * K,), -1, dtype=torch.int64, device=cuda_device)
+    row_of[perm[:T * K // 2]] = live
+    want_f, want_b = shared.float(), shared.float()
+    d_rw = torch.zeros(T, K, device=cuda_device)
+    for k in range(K):
+        r = row_of.view(T, K)[:, k]
+        have = (r >= 0).unsqueeze(1)
+        picked = y[r.clamp(min=0)].float()
+        want_f = torch.where(have, want_f + picked * w[:, k:k + 1], want_f)
+        want_b = torch.where(have, want_b + picked, want_b)
+        for c in range(6):
+            d_rw[:, k] = torch.where(have[:, 0], d_rw[:, k] + parts[r.clamp(min=0), c], d_rw[:, k])
+    junk = torch.randint(-3, rows + 3, (T * K,), generator=g, device=cuda_device).int()
+    junk[::7] = 2 ** 31 - 1
+    st = L.stream_ptr(cuda_device)
+    out = torch.empty_like(shared)
+    L.check(L.mok_fwd_epilogue_rows(shared.data_ptr(), y.data_ptr(), rank.data_ptr(), tok.data_ptr(), n.data_ptr(), w.data_ptr(),
+                                    junk.clone().data_ptr(), out.data_ptr(), T, H, K, rows, st), "fwd")
+    got_rw = torch.full((T, K), 9.0, device=cuda_device)
+    d_x = shared.clone()
+    L.check(L.mok_bwd_epilogue_rows(d_x.data_ptr(), y.data_ptr(), parts.data_ptr(), 6, rank.data_ptr(), tok.data_ptr(), n.data_ptr(),
+                                    junk.clone().data_ptr(), d_x.data_ptr(), got_rw.data_ptr(), T, H, K, rows, st), "bwd")
+    torch.cuda.synchronize()
+    assert torch.equal(out, want_f.bfloat16()) and torch.equal(d_x, want_b.bfloat16()) and torch.equal(got_rw, d_rw)
+
+
 def test_schedule_full_size_properties(cuda_device):
     """EP=8 x 16384 tokens x top-8 (the MXFP8 benchmark shape): every route of every peer that
     targets this rank appears exactly once, experts are 256-padded, rows past num_tokens are -1."""
