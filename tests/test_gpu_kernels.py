@@ -179,6 +179,26 @@ def test_schedule_full_size_properties(cuda_device):
 # ----------------------------------------------------------------------------------------
 # MXFP8 quantiser: bit-exact bytes
 # ----------------------------------------------------------------------------------------
+@pytest.mark.parametrize("E,M,N,skip", [(1, 128, 128, 0), (3, 256, 384, 0), (1, 128, 256, 16), (2, 384, 128, 16)])
+def test_quantize_outputs_on_a_16_byte_boundary(cuda_device, E, M, N, skip):
+    """Outputs that are only 16-byte aligned take the kernel with half-block stores: the same bytes."""
+    L, ops = _mok()._lib, _mok().ops
+    g = torch.Generator(device=cuda_device).manual_seed(M + N)
+    x = torch.randn(E, M, N, generator=g, device=cuda_device).bfloat16()
+    x[0, 0, :4] = torch.tensor([float("inf"), float("nan"), 0.0, -0.0])
+    want = [t.view(torch.uint8).reshape(-1) for t in ops.mxfp8_quantize(x, True, True)]
+    got = [torch.zeros(t.numel() + skip, dtype=torch.uint8, device=cuda_device) for t in want]
+    for normal, transposed in ((True, True), (True, False), (False, True)):
+        for t in got:
+            t.zero_()
+        p = [t.data_ptr() + skip for t in got]
+        L.check(L.mok_mxfp8_quantize(x.data_ptr(), E, M, N, *(p[:2] if normal else (None, None)), *(p[2:] if transposed else (None, None)),
+                                     L.stream_ptr(cuda_device)), "quantize")
+        torch.cuda.synchronize()
+        for k in (0, 1) * normal + (2, 3) * transposed:
+            assert torch.equal(got[k][skip:], want[k]), (normal, transposed, k)
+
+
 def test_quantize_matches_golden(cuda_device, golden_dir):
     mok = _mok()
     z = np.load(os.path.join(golden_dir, "quantize.npz"))
