@@ -192,7 +192,9 @@ GemmCall wgrad(const mok_layer_common& c, bool routed, const void* a, int m, con
 enum Stage { kStageGateUp, kStageDown, kStageDgradDown, kStageDgradGateUp, kStageWgrad };
 
 // One launch of a stage.  `calls` may hold shared-expert GEMMs, routed ones, or both (a joint launch, used on one
-// rank where the row movement does not run beside the shared expert).
+// rank where the row movement does not run beside the shared expert).  The routed tiles go first: they read what the
+// stage before left in L2 (16384 tokens, H=2048, I=768, 128 experts, top-8, forward: 1789 us, 1809 with the shared expert's
+// tiles first, 1791 in launches of their own).  Weight gradients are the exception, see there.
 int launch_stage(Stage stage, std::initializer_list<GemmCall> calls, const mok_layer_common& c, const PassCtx& x, int off, int limit,
                  cudaStream_t s) {
     bool routed = false, shared = false;
@@ -508,8 +510,8 @@ extern "C" int mok_fwd_bf16(const mok_fwd_bf16_args* a, void* stream) {
                                             a->gate_routed, a->up_routed, a->hidden_routed);
                 const GemmCall dn = down(c, d, true, limit, a->hidden_routed, d.MB, a->w_routed_down, a->y_routed);
                 if (with_shared) {
-                    MOK_TRY(launch_stage(kStageGateUp, {shared_gate_up, up}, c, x, off, limit, st));
-                    return launch_stage(kStageDown, {shared_down, dn}, c, x, off, limit, st);
+                    MOK_TRY(launch_stage(kStageGateUp, {up, shared_gate_up}, c, x, off, limit, st));
+                    return launch_stage(kStageDown, {dn, shared_down}, c, x, off, limit, st);
                 }
                 MOK_TRY(launch_stage(kStageGateUp, {up}, c, x, off, limit, st));
                 return launch_stage(kStageDown, {dn}, c, x, off, limit, st);
@@ -594,8 +596,8 @@ extern "C" int mok_bwd_bf16(const mok_bwd_bf16_args* a, void* stream) {
                 const GemmCall dgu = dgrad_gate_up(c, d, true, limit, a->d_gate_routed, a->d_up_routed, d.MB, a->w_routed_gate,
                                                    a->w_routed_up, a->d_x_routed);
                 if (with_shared) {
-                    MOK_TRY(launch_stage(kStageDgradDown, {sh_dgrad_down, dd}, c, x, off, limit, st));
-                    return launch_stage(kStageDgradGateUp, {sh_dgrad_gate_up, dgu}, c, x, off, limit, st);
+                    MOK_TRY(launch_stage(kStageDgradDown, {dd, sh_dgrad_down}, c, x, off, limit, st));
+                    return launch_stage(kStageDgradGateUp, {dgu, sh_dgrad_gate_up}, c, x, off, limit, st);
                 }
                 MOK_TRY(launch_stage(kStageDgradDown, {dd}, c, x, off, limit, st));
                 return launch_stage(kStageDgradGateUp, {dgu}, c, x, off, limit, st);
