@@ -157,9 +157,10 @@ __global__ void __launch_bounds__(kEpiThreads, 8) epilogue_rows_kernel(const Epi
     auto look_up = [&](int group, int buf) {
         if (kWeighted && !kStaged) return;
         for (int i = threadIdx.x; i < entries; i += kEpiThreads) {
-            const int route = group * entries + i;
+            const unsigned at = static_cast<unsigned>(group * entries) + i;        // the last group may end past the routes
+            const int route = static_cast<int>(at);
             int row = -1;
-            if (route < p.T * p.K) {
+            if (at < static_cast<unsigned>(p.T * p.K)) {
                 row = row_of_route(route);
                 if (kWeighted) {
                     s_w[buf * entries + i] = p.weights[route];

@@ -5,7 +5,7 @@
 // Forward, per macrobatch window (last window first, so window 0's activations are the ones
 // left in the buffers for backward — same contract as the reference megakernel):
 //   dispatch rows  ->  [gate|up GEMM + SwiGLU]  ->  down GEMM  ->  combine rows
-// plus the dense shared expert on the local tokens.
+// plus the dense shared expert on the local tokens (on one rank inside the GEMM launches of the first window).
 // Backward, per window (first window first; later windows replay dispatch + gate/up):
 //   reverse-combine (w * d_y)  ->  [dgrad down + SwiGLU backward + router-grad partials]
 //   ->  dgrad gate+up (one accumulator)  ->  reverse-dispatch (+ router grads)  ->  3 wgrads
