@@ -12,6 +12,7 @@ Deliberate differences from the reference:
 from __future__ import annotations
 
 import inspect
+import operator
 
 import torch
 
@@ -27,6 +28,7 @@ _EP_TEXT = "1, 2, 4, 8"
 # ------------------------------------------------------------------------------------------
 _EXACT = {"Tensor": (Tensor, torch.nn.Parameter), "int": (int,), "bool": (bool,), "list[int]": (list,),
           "float | None": (float, int, type(None))}
+_requires_grad = operator.attrgetter("requires_grad")
 
 
 class _EagerOp(torch.library.CustomOpDef):
@@ -34,8 +36,9 @@ class _EagerOp(torch.library.CustomOpDef):
 
     Measured on one B200 host: the dispatcher's Python kernels (autograd, mutation and alias bookkeeping) cost 50-85 us
     per operator call, more than the launches behind it; a forward + backward of the smallest layer spent 300 of its
-    470 us there.  The body is called directly only with plain tensors and arguments of exactly the declared types,
-    outside compilation, tracing, functorch transforms, forward-mode AD, dispatch / function modes and profiling, and
+    470 us there.  The body is called directly only with plain tensors that have memory of their own (which meta, zero and
+    functional tensors do not) and arguments of exactly the declared types, outside compilation, tracing, functorch
+    transforms, forward-mode AD, dispatch / function modes and profiling, and
     when no gradient could be asked of the operator; everything else goes through the dispatcher as before.  What the
     dispatcher does for such a call besides running the body, bumping the version of the tensors it writes, is done here."""
 
@@ -55,11 +58,16 @@ class _EagerOp(torch.library.CustomOpDef):
             return False
         if not self.mok_required <= len(args) <= len(self.mok_types):
             return False
-        grad = torch.is_grad_enabled()
         for a, exact in zip(args, self.mok_types):
-            if type(a) not in exact or (grad and exact[0] is Tensor and a.requires_grad):
+            if type(a) not in exact:
                 return False
-        return True
+        tensors = [args[i] for i in self.mok_tensors]
+        if torch.is_grad_enabled() and any(map(_requires_grad, tensors)):
+            return False
+        try:
+            return all(map(Tensor.data_ptr, tensors))
+        except RuntimeError:                                    # sparse and the like: no memory to point to
+            return False
 
 
 def _operator(name: str, mutates_args, schema: str | None = None):
@@ -69,6 +77,7 @@ def _operator(name: str, mutates_args, schema: str | None = None):
         params = list(inspect.signature(body).parameters.values())
         op.mok_body = body
         op.mok_types = tuple(_EXACT[p.annotation] for p in params)
+        op.mok_tensors = tuple(i for i, exact in enumerate(op.mok_types) if exact[0] is Tensor)
         op.mok_required = sum(p.default is inspect.Parameter.empty for p in params)
         op.mok_mutated = tuple(i for i, p in enumerate(params) if p.name in mutates_args)
         op.__class__ = _EagerOp

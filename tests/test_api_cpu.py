@@ -303,3 +303,18 @@ def test_eager_operators_skip_the_dispatcher_only_where_it_would_forward_the_cal
     inside = []
     torch.func.vmap(lambda row: inside.append(direct(row, 2.0, out)) or row)(torch.ones(2, 4))
     assert inside == [False]
+
+
+def test_operators_take_meta_tensors_to_their_shape_functions():
+    import mok
+    meta = lambda dtype, *shape: torch.empty(*shape, dtype=dtype, device="meta")  # noqa: E731
+    tables = mok.ops.schedule(meta(torch.int32, 2, 512, 4), 8, 8192, 0)
+    assert [tuple(t.shape) for t in tables] == [(8192,), (8192,), (1,), (8,)]
+    assert [tuple(t.shape) for t in mok.ops.schedule_local(meta(torch.int64, 512, 4), 8, 8192)] == [(8192,), (8192,), (1,), (8,)]
+    q = mok.ops.mxfp8_quantize(meta(torch.bfloat16, 3, 256, 384), True, True)
+    assert [tuple(t.shape) for t in q] == [(3, 256, 384), (6, 3, 32, 16), (3, 384, 256), (9, 2, 32, 16)]
+    experts, weights = mok.ops.router_topk(meta(torch.float32, 512, 8), 2)
+    assert experts.dtype == torch.int64 and weights.shape == (512, 2)
+    assert all(t.is_meta for t in (*tables, *q, experts, weights))
+    # an operator that writes: nothing but shapes is touched
+    assert mok.ops.barrier_all(meta(torch.int32, 4), [1], 0, meta(torch.int32, 1)) is None
