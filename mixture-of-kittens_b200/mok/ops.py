@@ -28,6 +28,9 @@ _EP_TEXT = "1, 2, 4, 8"
 # ------------------------------------------------------------------------------------------
 _EXACT = {"Tensor": (Tensor, torch.nn.Parameter), "int": (int,), "bool": (bool,), "list[int]": (list,),
           "float | None": (float, int, type(None))}
+# keys under which a caller's kernel for plain CUDA or CPU tensors can be registered
+_KERNEL_KEYS = ("CUDA", "CPU", "AutogradCUDA", "AutogradCPU", "Autograd", "AutocastCUDA", "AutocastCPU", "ADInplaceOrView",
+                "BackendSelect", "CompositeExplicitAutograd", "CompositeExplicitAutogradNonFunctional", "CompositeImplicitAutograd")
 _requires_grad = operator.attrgetter("requires_grad")
 
 
@@ -37,10 +40,11 @@ class _EagerOp(torch.library.CustomOpDef):
     Measured on one B200 host: the dispatcher's Python kernels (autograd, mutation and alias bookkeeping) cost 50-85 us
     per operator call, more than the launches behind it; a forward + backward of the smallest layer spent 300 of its
     470 us there.  The body is called directly only with plain tensors that have memory of their own (which meta, zero and
-    functional tensors do not) and arguments of exactly the declared types, outside compilation, tracing, functorch
-    transforms, forward-mode AD, dispatch / function modes and profiling, and
-    when no gradient could be asked of the operator; everything else goes through the dispatcher as before.  What the
-    dispatcher does for such a call besides running the body, bumping the version of the tensors it writes, is done here."""
+    functional tensors do not) and no pending negation, and arguments of exactly the declared types, outside compilation,
+    tracing, functorch transforms, forward-mode AD, dispatch / function modes and profiling, when no gradient could be
+    asked of the operator and no kernel was registered for it beside the body; everything else goes through the
+    dispatcher.  What the dispatcher does for such a call besides running the body, bumping the version of the tensors it
+    writes, is done here."""
 
     def __call__(self, *args, **kwargs):
         if torch.compiler.is_compiling() or kwargs or not self._forwards_only(args):
@@ -54,7 +58,8 @@ class _EagerOp(torch.library.CustomOpDef):
         c = torch._C
         if (c._len_torch_dispatch_stack() or c._len_torch_function_stack() or c._get_tracing_state() is not None
                 or c._functorch.peek_interpreter_stack() is not None or torch.autograd._profiler_enabled()
-                or torch.autograd.forward_ad._current_level >= 0):
+                or torch.autograd.forward_ad._current_level >= 0
+                or not torch.library._impls.isdisjoint(self.mok_other_kernels)):
             return False
         if not self.mok_required <= len(args) <= len(self.mok_types):
             return False
@@ -65,7 +70,7 @@ class _EagerOp(torch.library.CustomOpDef):
         if torch.is_grad_enabled() and any(map(_requires_grad, tensors)):
             return False
         try:
-            return all(map(Tensor.data_ptr, tensors))
+            return all(map(Tensor.data_ptr, tensors)) and not any(map(Tensor.is_neg, tensors))
         except RuntimeError:                                    # sparse and the like: no memory to point to
             return False
 
@@ -80,6 +85,7 @@ def _operator(name: str, mutates_args, schema: str | None = None):
         op.mok_tensors = tuple(i for i, exact in enumerate(op.mok_types) if exact[0] is Tensor)
         op.mok_required = sum(p.default is inspect.Parameter.empty for p in params)
         op.mok_mutated = tuple(i for i, p in enumerate(params) if p.name in mutates_args)
+        op.mok_other_kernels = frozenset("/".join(name.split("::") + [key]) for key in _KERNEL_KEYS) - torch.library._impls
         op.__class__ = _EagerOp
         return op
     return register

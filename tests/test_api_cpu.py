@@ -318,3 +318,41 @@ def test_operators_take_meta_tensors_to_their_shape_functions():
     assert all(t.is_meta for t in (*tables, *q, experts, weights))
     # an operator that writes: nothing but shapes is touched
     assert mok.ops.barrier_all(meta(torch.int32, 4), [1], 0, meta(torch.int32, 1)) is None
+
+
+def _add_one_behind_torchs_back(name):
+    """An operator whose body writes through a raw pointer, as the kernels do: torch sees nothing of the write."""
+    import ctypes
+    import mok
+
+    def add_one(x, out) -> None:
+        floats = ctypes.c_float * x.numel()
+        src, dst = floats.from_address(x.data_ptr()), floats.from_address(out.data_ptr())
+        for i in range(x.numel()):
+            dst[i] = src[i] + 1.0
+    add_one.__annotations__ = {"x": "Tensor", "out": "Tensor"}
+    return mok.ops._operator(f"mok_test::{name}", mutates_args=("out",), schema="(Tensor x, Tensor(a!) out) -> ()")(add_one)
+
+
+def test_eager_operators_leave_unusual_tensors_and_registered_kernels_to_the_dispatcher():
+    import mok
+    op = _add_one_behind_torchs_back("unusual")
+    x, out = torch.arange(4.0), torch.zeros(4)
+    negated = torch._neg_view(x)
+    assert negated.is_contiguous() and not op._forwards_only((negated, out))
+    op(negated, out)
+    assert torch.equal(out, 1 - x)                          # the negation is carried out first
+    for odd in (torch._efficientzerotensor(4), torch._to_functional_tensor(x), x.to_sparse(), torch.empty(0)):
+        assert not op._forwards_only((odd, out))
+    assert op._forwards_only((x, out))
+
+    calls = []
+    torch.library.register_kernel(op, "cpu", lambda x, out: calls.append("registered"))
+    op(x, out)
+    assert calls == ["registered"]
+
+    other = _add_one_behind_torchs_back("library")
+    lib = torch.library.Library("mok_test", "IMPL")
+    lib.impl("library", lambda x, out: calls.append("library"), "CPU")
+    other(x, out)
+    assert calls == ["registered", "library"]
