@@ -34,6 +34,23 @@ _KERNEL_KEYS = ("CUDA", "CPU", "AutogradCUDA", "AutogradCPU", "Autograd", "Autoc
 _requires_grad = operator.attrgetter("requires_grad")
 
 
+def _eager_state():
+    """What tells a plain eager call, or None on a torch that lacks one of these (private) names: then every call takes
+    the dispatcher."""
+    try:
+        c = torch._C
+        torch.autograd.forward_ad._current_level                # a module global: read anew on each call
+        if not isinstance(torch.library._impls, set):
+            return None
+        return (c._len_torch_dispatch_stack, c._len_torch_function_stack, c._get_tracing_state,
+                c._functorch.peek_interpreter_stack, torch.autograd._profiler_enabled, torch.library._impls)
+    except AttributeError:
+        return None
+
+
+_EAGER_STATE = _eager_state()
+
+
 class _EagerOp(torch.library.CustomOpDef):
     """A `torch.library.custom_op` that skips the dispatcher when the dispatcher would only forward the call.
 
@@ -55,11 +72,9 @@ class _EagerOp(torch.library.CustomOpDef):
         return result
 
     def _forwards_only(self, args) -> bool:
-        c = torch._C
-        if (c._len_torch_dispatch_stack() or c._len_torch_function_stack() or c._get_tracing_state() is not None
-                or c._functorch.peek_interpreter_stack() is not None or torch.autograd._profiler_enabled()
-                or torch.autograd.forward_ad._current_level >= 0
-                or not torch.library._impls.isdisjoint(self.mok_other_kernels)):
+        dispatch_modes, function_modes, tracing, transforms, profiling, kernels = _EAGER_STATE
+        if (dispatch_modes() or function_modes() or tracing() is not None or transforms() is not None or profiling()
+                or torch.autograd.forward_ad._current_level >= 0 or not kernels.isdisjoint(self.mok_other_kernels)):
             return False
         if not self.mok_required <= len(args) <= len(self.mok_types):
             return False
@@ -79,6 +94,8 @@ def _operator(name: str, mutates_args, schema: str | None = None):
     """`torch.library.custom_op` with `_EagerOp`'s short way in."""
     def register(body):
         op = torch.library.custom_op(name, body, mutates_args=mutates_args, schema=schema)
+        if _EAGER_STATE is None:
+            return op
         params = list(inspect.signature(body).parameters.values())
         op.mok_body = body
         op.mok_types = tuple(_EXACT[p.annotation] for p in params)
@@ -86,7 +103,10 @@ def _operator(name: str, mutates_args, schema: str | None = None):
         op.mok_required = sum(p.default is inspect.Parameter.empty for p in params)
         op.mok_mutated = tuple(i for i, p in enumerate(params) if p.name in mutates_args)
         op.mok_other_kernels = frozenset("/".join(name.split("::") + [key]) for key in _KERNEL_KEYS) - torch.library._impls
-        op.__class__ = _EagerOp
+        try:
+            op.__class__ = _EagerOp
+        except TypeError:                                       # a torch whose operators cannot change class
+            pass
         return op
     return register
 

@@ -356,3 +356,16 @@ def test_eager_operators_leave_unusual_tensors_and_registered_kernels_to_the_dis
     lib.impl("library", lambda x, out: calls.append("library"), "CPU")
     other(x, out)
     assert calls == ["registered", "library"]
+
+
+def test_operators_take_the_dispatcher_on_a_torch_without_the_names_the_short_way_needs(monkeypatch):
+    import mok
+    assert mok.ops._EAGER_STATE is not None
+    monkeypatch.delattr(torch._C._functorch, "peek_interpreter_stack")
+    assert mok.ops._eager_state() is None
+    monkeypatch.setattr(mok.ops, "_EAGER_STATE", None)
+    op = _add_one_behind_torchs_back("plain")
+    x, out = torch.arange(4.0), torch.zeros(4)
+    assert type(op) is torch.library.CustomOpDef
+    op(x, out)
+    assert torch.equal(out, x + 1)
