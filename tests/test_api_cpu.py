@@ -369,3 +369,19 @@ def test_operators_take_the_dispatcher_on_a_torch_without_the_names_the_short_wa
     assert type(op) is torch.library.CustomOpDef
     op(x, out)
     assert torch.equal(out, x + 1)
+
+
+def test_eager_operators_bump_the_version_of_what_they_write():
+    op = _add_one_behind_torchs_back("bump")
+    x, direct, dispatched = torch.arange(4.0), torch.zeros(4), torch.zeros(4)
+    assert op._forwards_only((x, direct))
+    op(x, direct)
+    op(x=x, out=dispatched)
+    assert torch.equal(direct, x + 1) and torch.equal(dispatched, x + 1)
+    assert direct._version == dispatched._version == 1
+    w = torch.ones(4, requires_grad=True)
+    saved = torch.ones(4)
+    loss = (w * saved).sum()
+    op(x, saved)                                            # overwrites what backward needs
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        loss.backward()
