@@ -100,28 +100,27 @@ __global__ void __launch_bounds__(256) epilogue_kernel(const uint4* __restrict__
     }
 }
 
-// Route -> schedule row, for the epilogues that gather routed rows straight from the GEMM output.  Entries of routes
-// without a row are left as they are: the reader checks every entry against the schedule itself.
-__global__ void __launch_bounds__(256) invert_rows_kernel(const int* __restrict__ peer_rank, const int* __restrict__ peer_token_idx,
-                                                          const int* __restrict__ num_tokens, int row_limit, int routes,
-                                                          int* __restrict__ route_row) {
-    pdl_wait();
-    const int n = min(*num_tokens, row_limit);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (peer_rank[i] < 0) continue;
-        const int r = peer_token_idx[i];
-        if (r >= 0 && r < routes) route_row[r] = i;
-    }
-}
-
 struct EpilogueRows {
     const uint4* shared_rows; const uint4* rows; uint4* out;     // out may be shared_rows itself
-    const int* route_row; const int* peer_rank; const int* peer_token_idx; const int* num_tokens;
+    int* route_row; const int* peer_rank; const int* peer_token_idx; const int* num_tokens;
     int row_limit;
     const float* weights;                                        // forward
     const float* partials; int partial_cols; float* d_router_weights;   // backward
     int T, vec_per_row, K;
 };
+
+// Route -> schedule row, for the epilogues that gather routed rows straight from the GEMM output.  Entries of routes
+// without a row are left as they are: the reader checks every entry against the schedule itself.  Launched dependently, so
+// its pointers come in a struct: loads through a const __restrict__ parameter may be moved ahead of the wait.
+__global__ void __launch_bounds__(256) invert_rows_kernel(const EpilogueRows p) {
+    pdl_wait();
+    const int n = min(*p.num_tokens, p.row_limit), routes = p.T * p.K;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        if (p.peer_rank[i] < 0) continue;
+        const int r = p.peer_token_idx[i];
+        if (r >= 0 && r < routes) p.route_row[r] = i;
+    }
+}
 
 // Same arithmetic as epilogue_kernel, but the k-th routed row of token t is rows[route_row[t*K+k]] (a route without a
 // row adds nothing); kWeighted = forward, else backward, which also sums each route's router-gradient partials in
@@ -589,10 +588,9 @@ extern "C" int mok_bwd_epilogue(const void* d_x_shared, const void* d_x_routed_b
 }
 
 namespace {
-int epilogue_rows(bool weighted, const mok::EpilogueRows& p, int32_t* route_row, cudaStream_t s) {
+int epilogue_rows(bool weighted, const mok::EpilogueRows& p, cudaStream_t s) {
     ProfScope prof(kSlotEpilogue, s, 2);
-    MOK_TRY(launch_kernel(mok::invert_rows_kernel, std::min(1024, (p.row_limit + 255) / 256), 256, 0, s, false, true, p.peer_rank,
-                          p.peer_token_idx, p.num_tokens, p.row_limit, p.T * p.K, route_row));
+    MOK_TRY(launch_kernel(mok::invert_rows_kernel, std::min(1024, (p.row_limit + 255) / 256), 256, 0, s, false, true, p));
     const int tokens = epi_tokens(p.vec_per_row, p.K), groups = (p.T + tokens - 1) / tokens;
     const bool staged = p.K <= kEpiMaxStaged;
     const size_t smem = staged ? static_cast<size_t>(2) * tokens * p.K * 8 : 0;
@@ -620,7 +618,7 @@ extern "C" int mok_fwd_epilogue_rows(const void* y_shared, const void* y_routed,
     p.row_limit = row_limit;
     p.weights = topk_weights;
     p.T = num_local_tokens; p.vec_per_row = hidden / 8; p.K = topk;
-    return epilogue_rows(true, p, route_row, static_cast<cudaStream_t>(stream));
+    return epilogue_rows(true, p, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int mok_bwd_epilogue_rows(const void* d_x_shared, const void* d_x_routed, const float* partials, int partial_cols,
@@ -642,5 +640,5 @@ extern "C" int mok_bwd_epilogue_rows(const void* d_x_shared, const void* d_x_rou
     p.row_limit = row_limit;
     p.partials = partials; p.partial_cols = partial_cols; p.d_router_weights = d_router_weights;
     p.T = num_local_tokens; p.vec_per_row = hidden / 8; p.K = topk;
-    return epilogue_rows(false, p, route_row, static_cast<cudaStream_t>(stream));
+    return epilogue_rows(false, p, static_cast<cudaStream_t>(stream));
 }
