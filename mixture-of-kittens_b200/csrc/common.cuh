@@ -40,10 +40,13 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Programmatic dependent launch.  Every kernel of the library calls pdl_wait() before it touches global memory: it
-// returns once the kernels ahead of it on the stream have finished and their writes are visible (at once without the
-// launch attribute).  From then on the next kernel's CTAs may be placed and run their prologue while this one runs and
-// drains.  Only shared memory, tensor memory and kernel parameters may be touched before it.
+// Programmatic dependent launch.  A kernel that is launched through launch_kernel calls pdl_wait() before it touches
+// global memory: it returns once the kernels ahead of it on the stream have finished and their writes are visible (at
+// once without the launch attribute).  From then on the next kernel's CTAs may be placed and run their prologue while
+// this one runs and drains.  Only shared memory, tensor memory and kernel parameters may be touched before it, and inputs
+// come in a struct of plain pointers (loads through const __restrict__ parameters may be moved ahead of the wait).
+// Kernels without the wait must never get the attribute and are launched with <<<>>>: all_gather_kernel, barrier_kernel,
+// epilogue_kernel, mxfp8_quantize_kernel, router_topk_kernel and router_topk_bwd_kernel.
 // The next kernel is let in after the wait, not at entry: let in at entry, a chain of short kernels piles up on the
 // SMs and the one that runs gets the slots the waiting ones left (scheduler of eight ranks, back to back: 29.5 us so,
 // 18.8 us with one kernel ahead at most).
