@@ -314,8 +314,8 @@ bool overlap_shared_expert() {
 
 class Pipeline {
 public:
-    Pipeline(cudaStream_t main, int chunks, int min_rows, int comm_sms)
-        : main_(main), chunks_(chunks), min_rows_(min_rows), comm_sms_(comm_sms) {
+    Pipeline(cudaStream_t main, bool one_rank, int chunks, int min_rows, int comm_sms)
+        : main_(main), one_rank_(one_rank), chunks_(chunks), min_rows_(min_rows), comm_sms_(comm_sms) {
         if (cudaGetDevice(&dev_) != cudaSuccess || dev_ < 0 || dev_ >= 64) {
             note_error_text("cudaGetDevice failed or device index >= 64");
             rc_ = MOK_ERR_CUDA;
@@ -342,11 +342,12 @@ public:
     Pipeline(const Pipeline&) = delete;
     Pipeline& operator=(const Pipeline&) = delete;
     int error() const { return rc_; }
-    // row movement runs on a side stream beside launches of the caller's stream
-    bool overlaps() const { return use_side_; }
-    // Programmatic dependence only where all launches of the pass are on one stream: with row movement on a side stream,
-    // a GEMM CTA that is placed early would hold an SM that mover CTAs could use.
-    PassCtx whole() const { PassCtx x; x.dependent = !use_side_; return x; }
+    // One rank and all launches of the pass on the caller's stream: stages may be joint launches, and launches depend
+    // programmatically.  With row movement on a side stream a GEMM CTA that is placed early would hold an SM that mover
+    // CTAs could use.  With several ranks a pass may be on one stream too (windows below two minibatches are not cut); it
+    // keeps separate, plain launches, as the chunked passes of several ranks do.
+    bool local() const { return one_rank_ && !use_side_; }
+    PassCtx whole() const { PassCtx x; x.dependent = local(); return x; }
 
     // side stream continues after everything enqueued on main so far / main after side
     int fork() { if (!use_side_) return MOK_OK; forked_ = true; return order(main_, side_); }
@@ -415,6 +416,7 @@ private:
         return cudaStreamWaitEvent(then, e, 0) == cudaSuccess ? MOK_OK : MOK_ERR_CUDA;
     }
     cudaStream_t main_;
+    bool one_rank_;
     cudaStream_t side_ = nullptr;
     int chunks_, min_rows_, comm_sms_;
     int dev_ = -1;
@@ -476,7 +478,7 @@ extern "C" int mok_fwd_bf16(const mok_fwd_bf16_args* a, void* stream) {
     MOK_TRY(fill_peers(combine_peers, a->combine_buffer_ptrs, d.W));
     const void* x_local = x_peers.p[d.rank];
     const int chunks = pipeline_chunks(c, std::min(d.MB, d.cap));
-    Pipeline pipe(s, chunks, c.minibatch_size, pipeline_comm_sms(c, chunks));
+    Pipeline pipe(s, c.ep_size == 1, chunks, c.minibatch_size, pipeline_comm_sms(c, chunks));
     const PassCtx whole = pipe.whole();    // launches outside the chunked pipeline cover their whole window on all SMs
     MOK_TRY(pipe.error());
     MOK_TRY(pipe.fork());
@@ -484,9 +486,9 @@ extern "C" int mok_fwd_bf16(const mok_fwd_bf16_args* a, void* stream) {
     const GemmCall shared_gate_up = gate_up(c, d, false, d.T, x_local, d.T, a->w_shared_gate, a->w_shared_up, a->gate_shared,
                                             a->up_shared, a->hidden_shared);
     const GemmCall shared_down = down(c, d, false, d.T, a->hidden_shared, d.T, a->w_shared_down, a->y_shared);
-    // shared expert on the local tokens.  Rows moved in one piece: in the launches of the first window.  Chunked: its
-    // gate|up GEMM runs beside the first dispatch chunk, its down projection beside the last combine chunk.
-    const bool joint = !pipe.overlaps();
+    // shared expert on the local tokens.  One rank, rows moved in one piece: in the launches of the first window.  Chunked:
+    // its gate|up GEMM runs beside the first dispatch chunk, its down projection beside the last combine chunk.
+    const bool joint = pipe.local();
     const bool shared_down_last = chunks > 1;
     if (!joint) {
         MOK_TRY(launch_stage(kStageGateUp, {shared_gate_up}, c, whole, 0, 0, s));
@@ -546,7 +548,7 @@ extern "C" int mok_bwd_bf16(const mok_bwd_bf16_args* a, void* stream) {
     const void* x_local = x_peers.p[d.rank];
     const int partial_cols = d.I / kBlockN * kEpiSplit;
     const int chunks = pipeline_chunks(c, std::min(d.MB, d.cap));
-    Pipeline pipe(s, chunks, c.minibatch_size, pipeline_comm_sms(c, chunks));
+    Pipeline pipe(s, c.ep_size == 1, chunks, c.minibatch_size, pipeline_comm_sms(c, chunks));
     const PassCtx whole = pipe.whole();    // launches outside the chunked pipeline cover their whole window on all SMs
     MOK_TRY(pipe.error());
     MOK_TRY(pipe.fork());
@@ -559,7 +561,7 @@ extern "C" int mok_bwd_bf16(const mok_bwd_bf16_args* a, void* stream) {
                                   wgrad(c, false, a->d_gate_shared, d.I, x_local, d.H, d.T, a->d_w_shared_gate, 0),
                                   wgrad(c, false, a->d_up_shared, d.I, x_local, d.H, d.T, a->d_w_shared_up, 0)};
     // shared expert: in the launches of the first window, or ahead of it to overlap the first reverse-combine chunk
-    const bool joint = !pipe.overlaps();
+    const bool joint = pipe.local();
     if (!joint) {
         MOK_TRY(launch_stage(kStageDgradDown, {sh_dgrad_down}, c, whole, 0, 0, s));
         MOK_TRY(launch_stage(kStageDgradGateUp, {sh_dgrad_gate_up}, c, whole, 0, 0, s));
@@ -782,7 +784,7 @@ extern "C" int mok_fwd_mxfp8(const mok_fwd_mxfp8_args* a, void* stream) {
     MOK_TRY(fill_peers(combine_peers, a->combine_buffer_ptrs, d.W));
     const void* x_local = x_peers.p[d.rank];
     const int chunks = pipeline_chunks(c, std::min(d.MB, d.cap));
-    Pipeline pipe(s, chunks, c.minibatch_size, pipeline_comm_sms(c, chunks));
+    Pipeline pipe(s, c.ep_size == 1, chunks, c.minibatch_size, pipeline_comm_sms(c, chunks));
     const PassCtx whole = pipe.whole();    // launches outside the chunked pipeline cover their whole window on all SMs
     MOK_TRY(pipe.error());
     MOK_TRY(pipe.fork());
@@ -844,7 +846,7 @@ extern "C" int mok_bwd_mxfp8(const mok_bwd_mxfp8_args* a, void* stream) {
     const void* x_local = x_peers.p[d.rank];
     const int partial_cols = d.I / kBlockN;
     const int chunks = pipeline_chunks(c, std::min(d.MB, d.cap));
-    Pipeline pipe(s, chunks, c.minibatch_size, pipeline_comm_sms(c, chunks));
+    Pipeline pipe(s, c.ep_size == 1, chunks, c.minibatch_size, pipeline_comm_sms(c, chunks));
     const PassCtx whole = pipe.whole();    // launches outside the chunked pipeline cover their whole window on all SMs
     MOK_TRY(pipe.error());
     MOK_TRY(pipe.fork());
