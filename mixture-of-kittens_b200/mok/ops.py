@@ -31,7 +31,7 @@ _EXACT = {"Tensor": (Tensor, torch.nn.Parameter), "int": (int,), "bool": (bool,)
 # keys under which a caller's kernel for plain CUDA or CPU tensors can be registered
 _KERNEL_KEYS = ("CUDA", "CPU", "AutogradCUDA", "AutogradCPU", "Autograd", "AutocastCUDA", "AutocastCPU", "ADInplaceOrView",
                 "BackendSelect", "CompositeExplicitAutograd", "CompositeExplicitAutogradNonFunctional", "CompositeImplicitAutograd")
-_requires_grad = operator.attrgetter("requires_grad")
+_requires_grad, _data_ptr, _is_neg = operator.attrgetter("requires_grad"), Tensor.data_ptr, Tensor.is_neg
 
 
 def _eager_state():
@@ -78,14 +78,17 @@ class _EagerOp(torch.library.CustomOpDef):
             return False
         if not self.mok_required <= len(args) <= len(self.mok_types):
             return False
-        for a, exact in zip(args, self.mok_types):
-            if type(a) not in exact:
+        types = tuple(map(type, args))
+        if types not in self.mok_accepted:
+            if not all(t in exact for t, exact in zip(types, self.mok_types)):
                 return False
-        tensors = [args[i] for i in self.mok_tensors]
+            if len(self.mok_accepted) < 64:                     # tensors and parameters mix in a few ways
+                self.mok_accepted.add(types)
+        tensors = self.mok_tensors(args)
         if torch.is_grad_enabled() and any(map(_requires_grad, tensors)):
             return False
         try:
-            return all(map(Tensor.data_ptr, tensors)) and not any(map(Tensor.is_neg, tensors))
+            return all(map(_data_ptr, tensors)) and not any(map(_is_neg, tensors))
         except RuntimeError:                                    # sparse and the like: no memory to point to
             return False
 
@@ -99,7 +102,9 @@ def _operator(name: str, mutates_args, schema: str | None = None):
         params = list(inspect.signature(body).parameters.values())
         op.mok_body = body
         op.mok_types = tuple(_EXACT[p.annotation] for p in params)
-        op.mok_tensors = tuple(i for i, exact in enumerate(op.mok_types) if exact[0] is Tensor)
+        op.mok_accepted = set()
+        at = [i for i, exact in enumerate(op.mok_types) if exact[0] is Tensor]
+        op.mok_tensors = operator.itemgetter(*at) if len(at) > 1 else lambda args: (args[at[0]],)
         op.mok_required = sum(p.default is inspect.Parameter.empty for p in params)
         op.mok_mutated = tuple(i for i, p in enumerate(params) if p.name in mutates_args)
         op.mok_other_kernels = frozenset("/".join(name.split("::") + [key]) for key in _KERNEL_KEYS) - torch.library._impls
