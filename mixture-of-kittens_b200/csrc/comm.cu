@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(256) invert_rows_kernel(const EpilogueRows p) 
 // row adds nothing); kWeighted = forward, else backward, which also sums each route's router-gradient partials in
 // column order.  `out` may be `shared_rows` itself (the backward pass sums in place: every element is read by the
 // thread that writes it, before it writes), so neither is restrict.
-// HBM-bound: (K+2)*H*2 bytes per token.  A block takes a whole token (several where H < 2048), so that a row is read in
-// one piece; while it streams one, it looks up and checks the rows of its next one.
+// HBM-bound: (K+2)*H*2 bytes per token.  A block takes a whole token (several where H <= 1024; from there to 2048 one, with
+// idle lanes), so that a row is read in one piece; while it streams one, it looks up and checks the rows of its next one.
 // Occupancy decides (2048 threads per SM at 32 registers; 1024 threads with four rows in flight each: 160 us).
 // 16384 tokens, H=2048, top-8, with the inversion of the table: 133 us, as with a separate clear and the table walked by
 // every thread (132), 188 with a token cut into 1 KB slices, one per warp.  Where router gradients are summed, by the

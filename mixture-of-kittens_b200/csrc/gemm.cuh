@@ -66,10 +66,11 @@ struct GemmParams {
 
 // A launch: up to six GEMMs of one kind (same operand layouts and epilogue), whose tiles form one list that the
 // persistent CTAs walk.  The dense shared expert and the routed experts of a pass, or the six weight gradients of a
-// backward pass, run as one launch: one ramp and one ragged last wave instead of one each, 4 GEMM launches per BF16
-// training step instead of 14.  One B200, separate -> joint: 2816 tokens, H=1792, I=1280, 24 experts, top-5, training
-// step 1040 -> 982 us; 512 tokens, H=2048, I=768, 128 experts, top-8, forward 390 -> 370 us; 8192 tokens in three windows,
-// training step 2616 -> 2544 us; 16384 tokens: within 1 %.
+// backward pass, run as one launch: one ramp and one ragged last wave instead of one each, 5 GEMM launches per BF16
+// training step instead of 14.  One B200, separate -> joint launches, timed in turn: 2816 tokens, H=1792, I=1280, 24 experts,
+// top-5, training step 1003 -> 948 us; H=2048, I=768, 128 experts, top-8, forward of 512 tokens 376 -> 354 us, of 16384
+// tokens 1732 -> 1679 us; no difference beyond the spread of 8192 tokens in three windows (2.54 ms) and of 16384 tokens,
+// H=4096, I=1536, 8 experts, top-6, training steps (11.32 -> 11.25 ms).
 constexpr int kMaxGemms = 6;
 struct GemmBatch {
     CUtensorMap a0[kMaxGemms], b0[kMaxGemms];

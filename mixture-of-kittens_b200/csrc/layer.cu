@@ -192,9 +192,10 @@ GemmCall wgrad(const mok_layer_common& c, bool routed, const void* a, int m, con
 enum Stage { kStageGateUp, kStageDown, kStageDgradDown, kStageDgradGateUp, kStageWgrad };
 
 // One launch of a stage.  `calls` may hold shared-expert GEMMs, routed ones, or both (a joint launch, used on one
-// rank where the row movement does not run beside the shared expert).  The routed tiles go first: they read what the
-// stage before left in L2 (16384 tokens, H=2048, I=768, 128 experts, top-8, forward: 1789 us, 1809 with the shared expert's
-// tiles first, 1791 in launches of their own).  Weight gradients are the exception, see there.
+// rank where the row movement does not run beside the shared expert).  The order of the two makes
+// no difference beyond the spread (16384 tokens, H=2048, I=768, 128 experts, top-8, forward: 1678 and 1680 us in two runs,
+// 1689 and 1678 with the shared expert's tiles first); the routed tiles, which read what the stage before left in L2, go
+// first.  Weight gradients are the exception, see there.
 int launch_stage(Stage stage, std::initializer_list<GemmCall> calls, const mok_layer_common& c, const PassCtx& x, int off, int limit,
                  cudaStream_t s) {
     bool routed = false, shared = false;
