@@ -4,20 +4,27 @@
 // "thread-major" over 1024 virtual threads, peers are interleaved round-robin inside an expert,
 // experts are padded to 256 rows.
 //
-// The reference rescans every peer's routes 2*El times.  Here every route is read twice; a chunk is the routes of 4
-// virtual threads of one peer, a block handles 8 consecutive chunks, a warp one:
+// The reference rescans every peer's routes 2*El times.  Here every route is read three times, or twice with the scan
+// kernel below; a chunk is the routes of 4 virtual threads of one peer, a block handles 8 consecutive chunks, a warp one:
 //   count   every block histograms its routes per local expert in shared memory   -> block_hist[peer][block][expert]
 //           and all blocks together clear the tables
 //   place   every block sums block_hist into the expert totals of every peer and its own start offsets, counts its
 //           chunks again in shared memory for the offsets of its warps, then each warp walks its routes in order, ranks
 //           equal experts inside the warp with match.any, and writes the slots
-// The place blocks re-read W*32*El counts each.  Above W*El = 256 that costs more than one more launch (back to back,
-// 16384 tokens, top-8: 8 ranks with 32 experts each 18.8 us against 19.0 with the scan, with 64 each 40 against 21), so
-// larger problems run a scan kernel in between that turns the chunk counts into offsets once:
+// The place blocks re-read W*32*El counts each, one (rank, expert) pair per thread up to W*El = 256.  Larger problems run a
+// scan kernel in between that turns the chunk counts into offsets once, and launch all three kernels plainly:
 //   scan    one warp per (expert, peer): exclusive offsets of the 256 chunks and the total   -> cnt[expert][peer]
-// Algorithmic traffic: 2 * W*T*K*4 B of route reads + 2 * capacity * 4 B of table writes; at these sizes launches and
-// the latency of dependent loads decide (8 ranks x 32 experts 23.3 us and one rank x 128 experts 21.2 us before, 18.8 and
-// 15.2 now; 8 ranks x 256 experts 18.9, now 17.0).  Routes are read as int32 or, on one rank, as the caller's int64.
+// Calls back to back on one stream, top-8, us with two kernels / with three, one B200:
+//   W*El                          64          256          320          384          512
+//   1 rank,    512 tokens    7.4 / 16.4   7.8 / 16.4  10.4 / 18.4  10.7 / 17.4  11.0 / 17.4
+//   1 rank,  16384 tokens   15.7 / 22.6  16.0 / 22.6  18.8 / 24.6  19.1 / 22.9  18.8 / 24.6
+//   8 ranks,   512 tokens    9.0 / 16.4   9.6 / 16.6  10.8 / 18.4  11.6 / 18.4  11.1 / 18.4
+//   8 ranks, 16384 tokens   20.1 / 26.6  20.2 / 26.6  21.6 / 26.7  22.4 / 26.6  41.6 / 26.6
+// So the line, where a thread takes its second pair, is on the near side of a steep rise that comes between 384 and 512.
+// Algorithmic traffic: W*T*K ids of 4 or 8 B, three times or twice, + 2 * capacity * 4 B of table writes; at these sizes
+// launches and the latency of dependent loads decide (before, with three kernels always: 8 ranks x 32 experts 30.7 us, now
+// 20.4; one rank x 128 experts 28.7, now 15.7, or 18.1 from int64 ids without the cast in front; 8 ranks x 256 experts 36.2,
+// now 30.4).  Routes are read as int32 or, on one rank, as the caller's int64.
 #include <algorithm>
 #include <atomic>
 
