@@ -48,3 +48,13 @@ def test_kernels_launched_dependently_wait_and_take_no_restrict_pointers():
     for name in waiting:
         params, body = found[name]
         assert "__restrict__" not in params and "__ldg" not in body and ".nc" not in body, name
+
+
+def test_kernels_without_the_wait_are_launched_plainly():
+    """launch_kernel can let a kernel start before the one ahead has finished; it is for kernels that call pdl_wait only."""
+    found = kernels()
+    plain = {name for name, (_, body) in found.items() if "pdl_wait()" not in body}
+    for _, text in _sources():
+        for m in re.finditer(r"\b(%s)\b" % "|".join(sorted(plain)), text):
+            statement = text[max(text.rfind(c, 0, m.start()) for c in ";{}") + 1:text.index(";", m.end()) if ";" in text[m.end():] else None]
+            assert "launch_kernel" not in statement and not re.match(r"\s*auto\s*\*\s*kern", statement), m.group(1)
