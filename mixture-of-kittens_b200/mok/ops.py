@@ -49,6 +49,8 @@ def _eager_state():
 
 
 _EAGER_STATE = _eager_state()
+_dispatch_modes, _function_modes, _tracing, _transforms, _profiling, _registered = _EAGER_STATE or (None,) * 6
+_forward_ad, _grad_enabled = torch.autograd.forward_ad, torch.is_grad_enabled
 
 
 class _EagerOp(torch.library.CustomOpDef):
@@ -72,25 +74,27 @@ class _EagerOp(torch.library.CustomOpDef):
         return result
 
     def _forwards_only(self, args) -> bool:
-        dispatch_modes, function_modes, tracing, transforms, profiling, kernels = _EAGER_STATE
-        if (dispatch_modes() or function_modes() or tracing() is not None or transforms() is not None or profiling()
-                or torch.autograd.forward_ad._current_level >= 0 or not kernels.isdisjoint(self.mok_other_kernels)):
-            return False
-        if not self.mok_required <= len(args) <= len(self.mok_types):
+        if (_dispatch_modes() or _function_modes() or _tracing() is not None or _transforms() is not None or _profiling()
+                or _forward_ad._current_level >= 0 or not _registered.isdisjoint(self.mok_other_kernels)):
             return False
         types = tuple(map(type, args))
-        if types not in self.mok_accepted:
-            if not all(t in exact for t, exact in zip(types, self.mok_types)):
-                return False
-            if len(self.mok_accepted) < 64:                     # tensors and parameters mix in a few ways
-                self.mok_accepted.add(types)
+        if types not in self.mok_accepted and not self._accepts(types):
+            return False
         tensors = self.mok_tensors(args)
-        if torch.is_grad_enabled() and any(map(_requires_grad, tensors)):
+        if _grad_enabled() and any(map(_requires_grad, tensors)):
             return False
         try:
             return all(map(_data_ptr, tensors)) and not any(map(_is_neg, tensors))
         except RuntimeError:                                    # sparse and the like: no memory to point to
             return False
+
+    def _accepts(self, types) -> bool:
+        if not (self.mok_required <= len(types) <= len(self.mok_types)
+                and all(t in exact for t, exact in zip(types, self.mok_types))):
+            return False
+        if len(self.mok_accepted) < 64:                         # tensors and parameters mix in a few ways
+            self.mok_accepted.add(types)
+        return True
 
 
 def _operator(name: str, mutates_args, schema: str | None = None):
