@@ -588,15 +588,23 @@ extern "C" int mok_bwd_epilogue(const void* d_x_shared, const void* d_x_routed_b
 }
 
 namespace {
+// Routed rows up to which the two kernels are launched dependently: about what L2 holds.  A short epilogue gains the launch
+// latency, a long one runs more slowly than after a plain launch (probably because its first CTAs, placed beside GEMM CTAs
+// that drain, keep the SMs at the GEMM's shared-memory carve-out, with little L1).  Dependent against plain on one B200, whole
+// passes in turn: 0.5 MB of rows 116.5 against 117.9 us, 17 MB 367 against 369, 50 MB 975 against 977; 235 MB 1141 against 1138,
+// 0.6 GB 1466 against 1454 and 1469 against 1457, 1.9 GB 24.98 against 24.94 ms.
+constexpr size_t kEpiDependentBytes = size_t{128} << 20;
+
 int epilogue_rows(bool weighted, const mok::EpilogueRows& p, cudaStream_t s) {
     ProfScope prof(kSlotEpilogue, s, 2);
-    MOK_TRY(launch_kernel(mok::invert_rows_kernel, std::min(1024, (p.row_limit + 255) / 256), 256, 0, s, false, true, p));
+    const bool dependent = static_cast<size_t>(p.T) * p.K * p.vec_per_row * sizeof(uint4) <= kEpiDependentBytes;
+    MOK_TRY(launch_kernel(mok::invert_rows_kernel, std::min(1024, (p.row_limit + 255) / 256), 256, 0, s, false, dependent, p));
     const int tokens = epi_tokens(p.vec_per_row, p.K), groups = (p.T + tokens - 1) / tokens;
     const bool staged = p.K <= kEpiMaxStaged;
     const size_t smem = staged ? static_cast<size_t>(2) * tokens * p.K * 8 : 0;
     auto* kern = weighted ? (staged ? mok::epilogue_rows_kernel<true, true> : mok::epilogue_rows_kernel<true, false>)
                           : (staged ? mok::epilogue_rows_kernel<false, true> : mok::epilogue_rows_kernel<false, false>);
-    return launch_kernel(kern, std::min(groups, 16 * device_sm_count()), kEpiThreads, smem, s, false, true, p);
+    return launch_kernel(kern, std::min(groups, 16 * device_sm_count()), kEpiThreads, smem, s, false, dependent, p);
 }
 }  // namespace
 

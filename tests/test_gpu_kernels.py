@@ -110,7 +110,8 @@ def test_schedule_int32_and_int64_ids_and_alignment(cuda_device, W, T, K, El, sk
                 assert np.array_equal(r, t.cpu().numpy()), (dtype, rank)
 
 
-@pytest.mark.parametrize("T,H,K", [(512, 256, 2), (768, 1280, 33), (512, 2304, 5), (3, 8, 300), (5, 24, 1025)])
+@pytest.mark.parametrize("T,H,K", [(512, 256, 2), (768, 1280, 33), (512, 2304, 5), (3, 8, 300), (5, 24, 1025),
+                                   (4096, 2048, 8), (4097, 2048, 8)])      # the largest dependent launch, the smallest plain one
 def test_epilogue_rows_checks_every_route_entry(cuda_device, T, H, K):
     """The route table is not cleared before it is filled: whatever an entry of a route without a row holds (another
     row, a padding row, anything out of range), the route adds nothing.  Sums are in k order, so the result is exact."""
